@@ -237,6 +237,7 @@ static void free_graph_arrays(gs_graph* g) {
     gs_stream_close(g);
     pr_layout_free(g);
     pb_layout_free(g);
+    rl_layout_free(g);
     for (void* p : {(void*)g->d_rec, (void*)g->d_items, (void*)g->d_tile_off, (void*)g->d_tile_rc,
                     (void*)g->d_degree, (void*)g->d_runs, (void*)g->d_runs_lpt, (void*)g->d_units,
                     (void*)g->d_runs_blk, (void*)g->d_units_blk, (void*)g->d_runs_blk2, (void*)g->d_units_blk2})

@@ -131,6 +131,29 @@ struct gs_pb_layout {
     bool built = false;
 };
 
+// PageRank row lists (gs_pr_rows.cu): every destination's sources, cut into
+// segments, 32 segments of one length to a slice, slices grouped into units;
+// panels are consecutive ranges of the sources in falling order of use.
+constexpr uint32_t kRlMaxPanels = 64;
+struct gs_rl_unit {              // slices [slice, slice + n_slices): `steps` x 32 16-byte groups from group off x 32 on
+    uint32_t slice, n_slices, off, steps;
+};
+struct gs_rl_layout {
+    uint32_t* d_ent = nullptr;       // entries, transposed by slice
+    uint32_t* d_row = nullptr;       // destination vertex of every segment (~0: none), then
+    uint8_t* d_n4 = nullptr;         // the steps of every slice
+    float* d_x = nullptr;            // x in source order, written at the start of a sweep, then
+    uint32_t* d_src = nullptr;       // the vertex of every source position,
+    gs_rl_unit* d_units = nullptr;   // the units,
+    unsigned int* d_tick = nullptr;  // and a unit ticket per panel and the CTAs finished
+    uint32_t n_src = 0, n_panels = 0, grid = 0;
+    uint32_t unit_beg[kRlMaxPanels + 1] = {};   // units of each panel
+    uint32_t home_beg[kRlMaxPanels + 1] = {};   // CTAs that start on each panel
+    uint64_t n_entries = 0;
+    bool built = false;
+    bool refused = false;            // another layout sweeps this graph faster
+};
+
 struct gs_streamer;   // pinned-host record stream of a graph (gs_stream.cu)
 struct gs_seglists;   // double-buffered entry lists of segment sweeps (gs_stream.cu)
 
@@ -197,7 +220,8 @@ struct gs_graph {
     bool nonisolated_known = false;
     SegView seg;                      // set during segment sweeps
     gs_pr_layout pr;                  // row-slice PageRank layout (serving, batches, smaller graphs)
-    gs_pb_layout pb;                  // propagation-blocked PageRank layout (gs_run on large graphs)
+    gs_pb_layout pb;                  // propagation-blocked PageRank layout (serving, gs_run on large graphs without hubs)
+    gs_rl_layout rl;                  // row-list PageRank layout (gs_run)
     gs_streamer* stream = nullptr;    // non-null: records stay in host memory
     gs_seglists* lists = nullptr;     // segment entry lists of segment sweeps
     std::vector<gs_tile_run> h_runs;  // host copies of the run and unit tables
@@ -327,6 +351,13 @@ gs_status pr_slice_sweep(gs_graph* g, cudaStream_t stream, const float* x, float
 gs_status pr_finalize_launch(gs_ctx* ctx, cudaStream_t stream, float* x, float* y, float* r, const int32_t* deg,
                              uint64_t N, uint64_t V, int compat);
 gs_status pr_sweep_launch(gs_state* s);
+// Row-list PageRank (gs_pr_rows.cu): whether the layout fits, building it
+// (rl.built stays false, rl.refused is set, when another one is faster on
+// this graph) and freeing it, one sweep.
+bool rl_layout_wanted(const gs_graph* g);
+gs_status rl_layout_build(gs_graph* g);
+void rl_layout_free(gs_graph* g);
+gs_status rl_launch(gs_state* s);
 // Propagation-blocked PageRank (gs_pr_blocked.cu): whether the layout is worth
 // building for this graph (and fits), building and freeing it, one sweep.
 bool pb_layout_wanted(const gs_graph* g);

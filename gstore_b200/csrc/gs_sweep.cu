@@ -603,17 +603,22 @@ gs_status pr_init(gs_state* s) {
     ctx->launches++;
     GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_r, 0, g->N * 4, ctx->stream));
     if (s->d_error) GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_error, 0, sizeof(uint64_t), ctx->stream));
-    // resident graphs sweep the propagation-blocked layout when it is worth
+    // resident graphs sweep the row lists when they fit and are the fastest
+    // (rl_worth), else the propagation-blocked layout when it is worth
     // building and fits, else the row-slice layout (each built once per graph)
-    if (!g->stream && g->E && !g->pb.built && !g->pr.built) {
-        if (pb_layout_wanted(g)) GS_TRY(pb_layout_build(g));
-        else GS_TRY(pr_layout_build(g));
+    if (!g->stream && g->E && !g->rl.built && !g->pb.built) {
+        if (!g->rl.refused && rl_layout_wanted(g)) GS_TRY(rl_layout_build(g));
+        if (!g->rl.built && !g->pr.built) {
+            if (pb_layout_wanted(g)) GS_TRY(pb_layout_build(g));
+            else GS_TRY(pr_layout_build(g));
+        }
     }
     return GS_OK;
 }
 
 gs_status pr_sweep_launch(gs_state* s) {
     gs_graph* g = s->g;
+    if (!g->seg.list && g->rl.built) return rl_launch(s);
     if (!g->seg.list && g->pb.built) return pb_launch(s);
     if (!g->seg.list && g->pr.built) return pr_slice_launch(s);
     if (g->stream) {

@@ -33,6 +33,13 @@ gs_status gs_dev_alloc(gs_ctx* ctx, void** ptr, size_t bytes) {
         gs_pool_clear(ctx);
         e = cudaMalloc(ptr, bytes);
     }
+    if (e == cudaErrorMemoryAllocation && ctx && !ctx->adj_graphs.empty()) {
+        // adjacency lists only save time: drop them, try once more
+        cudaGetLastError();
+        gs_adj_release(ctx);
+        gs_pool_clear(ctx);
+        e = cudaMalloc(ptr, bytes);
+    }
     if (e != cudaSuccess) {
         *ptr = nullptr;
         return gs_cuda_fail(ctx, e, "cudaMalloc");
@@ -238,6 +245,9 @@ static void free_graph_arrays(gs_graph* g) {
     pr_layout_free(g);
     pb_layout_free(g);
     rl_layout_free(g);
+    gs_adj_free(g);
+    auto& lists = g->ctx->adj_graphs;
+    lists.erase(std::remove(lists.begin(), lists.end(), g), lists.end());
     for (void* p : {(void*)g->d_rec, (void*)g->d_items, (void*)g->d_tile_off, (void*)g->d_tile_rc,
                     (void*)g->d_degree, (void*)g->d_runs, (void*)g->d_runs_lpt, (void*)g->d_units,
                     (void*)g->d_runs_blk, (void*)g->d_units_blk, (void*)g->d_runs_blk2, (void*)g->d_units_blk2})
@@ -906,6 +916,13 @@ gs_status gs_finalize(gs_state* s, int64_t* frontier_out, int* done_out) {
 gs_status gs_run(gs_state* s, int64_t* steps_out) {
     if (!s) return GS_ERR_ARG;
     int64_t steps = 0;
+    if (s->step == 0 && !s->swept && !s->done) {
+        // a whole query: on the graph's adjacency lists once it has them (the
+        // credits are the sweeps of the grid that each takes without)
+        if (s->algo == GS_ALGO_BFS && gs_adj_ready(s->g, 4)) GS_TRY(bfs_adj_run(s, &steps));
+        if (s->algo == GS_ALGO_KCORE && gs_adj_ready(s->g, 4)) GS_TRY(kcore_adj_run(s, &steps));
+        if (s->algo == GS_ALGO_WCC) gs_adj_ready(s->g, 3);
+    }
     if (s->algo == GS_ALGO_KCORE && s->step == 0 && !s->done) {
         // kcore_mmap runs one iteration_finalize before the first sweep
         // (gstore.cpp:2725-2726).
@@ -989,11 +1006,12 @@ gs_status gs_bfs_stats(gs_state* s, uint64_t* edges_in_component, uint64_t* swep
     if (level_counts)
         for (int l = 0; l < nl && l < max_levels; ++l) level_counts[l] = s->level_counts[l];
     if (swept_records) {
-        const int nh = std::min(std::min(nl, max_levels), std::min(s->n_act_hist, 256));
+        const int nh = std::min(std::min(nl, max_levels), 255);
         if (nh > 0) {
             gs_ctx* ctx = s->g->ctx;
             const size_t nw = s->g->nw;
             std::vector<uint8_t> hist((size_t)nh * nw);
+            GS_TRY(gs_level_windows(s, nh));
             GS_CHECK_CUDA(ctx, cudaMemcpyAsync(hist.data(), s->d_act_hist, hist.size(), cudaMemcpyDeviceToHost,
                                                ctx->stream));
             GS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

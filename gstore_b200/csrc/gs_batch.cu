@@ -49,44 +49,6 @@ using namespace gsops;
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr uint64_t kBarrierNs = 4000000000ull;   // 4 s
-
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Grid-wide barrier of a cooperative launch.  bar[0] counts arrivals, bar[1]
-// is the generation.  False when the wait gave up or another CTA failed.
-__device__ bool grid_barrier(unsigned int* bar, int* err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned int* vgen = bar + 1;
-        const unsigned int gen = *vgen;
-        __threadfence();
-        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            const uint64_t t0 = global_ns();
-            while (*vgen == gen) {
-                if (*(volatile int*)err) break;
-                if (global_ns() - t0 > kBarrierNs) {
-                    atomicOr(err, 1);
-                    break;
-                }
-                __nanosleep(100);
-            }
-        }
-        __threadfence();
-        ok = *(volatile int*)err == 0;
-    }
-    __syncthreads();
-    return ok != 0;
-}
 
 // ------------------------------------------------------------ MS-BFS ----
 template <class W>
@@ -339,8 +301,10 @@ struct BQuery {
     const gs_tile_run* runs;
     const gs_unit* units;
     const uint32_t* rec;
-    uint64_t R;
+    uint64_t R;                  // draws of a sweep: runs, or kAdjWords-word blocks of the adjacency lists
     uint64_t words;              // N / 32
+    const uint32_t* off;         // k-core: the graph's adjacency lists (null: sweep the tiles)
+    const uint32_t* adj;
     uint32_t nw;
     int algo;
     int k;
@@ -354,6 +318,10 @@ struct BQuery {
 };
 
 constexpr int kMaxBatch = 64;
+constexpr uint64_t kAdjWords = 32;   // vertex words a CTA takes at a time (k-core on adjacency lists)
+constexpr uint32_t kAdjLane = 64;    // longest list a lane walks alone
+constexpr uint32_t kAdjWarp = 1024;  // longest list a warp walks alone
+constexpr int kAdjLong = 64;         // longer ones wait for the whole CTA, so many at a time
 constexpr int kMsCtasPerSm = 4;   // multi-source BFS launches
 constexpr int kWkCtasPerSm = 8;   // WCC / k-core launches (their sweeps wait on dependent loads)
 
@@ -383,7 +351,8 @@ __device__ __forceinline__ int find_query(const uint64_t* pre, int n, uint64_t x
 __global__ void __launch_bounds__(kThreads) wk_batch_kernel(BatchArgs a) {
     __shared__ uint64_t run_pre[kMaxBatch + 1], word_pre[kMaxBatch + 1];
     __shared__ int act_q[kMaxBatch];
-    __shared__ int n_act;
+    __shared__ int n_act, n_long;
+    __shared__ uint2 long_row[kAdjLong];
     __shared__ unsigned long long done_mask, s_run;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t gwarp = (uint64_t)blockIdx.x * kWarps + warp;
@@ -466,7 +435,46 @@ __global__ void __launch_bounds__(kThreads) wk_batch_kernel(BatchArgs a) {
             const int ai = find_query(run_pre, n_act, x);
             const BQuery& q = a.q[act_q[ai]];
             const gs_tile_run run = q.runs[x - run_pre[ai]];
-            if (q.algo == GS_ALGO_KCORE) {
+            if (q.algo == GS_ALGO_KCORE && q.off) {
+                // the lists of the vertices removed this round, instead of every record
+                const uint64_t w0 = (x - run_pre[ai]) * kAdjWords;
+                if (threadIdx.x == 0) n_long = 0;
+                __syncthreads();
+                for (uint64_t w = w0 + warp; w < w0 + kAdjWords && w < q.words; w += kWarps) {
+                    const uint32_t rw = __ldcg(q.removed + w);
+                    if (!rw) continue;   // uniform
+                    const bool gone = rw >> lane & 1u;
+                    const uint32_t b = gone ? __ldg(q.off + w * 32 + lane) : 0u;
+                    const uint32_t e = gone ? __ldg(q.off + w * 32 + lane + 1) : 0u;
+                    if (e - b <= kAdjLane)
+                        for (uint32_t i = b; i < e; i += 4) {
+                            uint32_t n[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) n[j] = i + j < e ? __ldg(q.adj + i + j) : ~0u;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (n[j] != ~0u) atomicSub(q.deg + n[j], 1);
+                        }
+                    uint32_t more = __ballot_sync(kFull, e - b > kAdjLane);
+                    while (more) {
+                        const uint32_t l = __ffs(more) - 1;
+                        more &= more - 1;
+                        const uint32_t lb = __shfl_sync(kFull, b, l), le = __shfl_sync(kFull, e, l);
+                        int at = kAdjLong;
+                        if (le - lb > kAdjWarp && lane == 0) at = atomicAdd(&n_long, 1);
+                        at = __shfl_sync(kFull, at, 0);
+                        if (at < kAdjLong) {
+                            if (lane == 0) long_row[at] = make_uint2(lb, le);
+                            continue;
+                        }
+                        for (uint32_t i = lb + lane; i < le; i += 32) atomicSub(q.deg + __ldg(q.adj + i), 1);
+                    }
+                }
+                __syncthreads();
+                for (int k = 0; k < min(n_long, kAdjLong); ++k)
+                    for (uint32_t i = long_row[k].x + threadIdx.x; i < long_row[k].y; i += kThreads)
+                        atomicSub(q.deg + __ldg(q.adj + i), 1);
+            } else if (q.algo == GS_ALGO_KCORE) {
                 const KcoreOpL2 op{q.deg, q.removed, q.act + p * q.nw};
                 for (uint32_t ui = run.unit_beg + warp; ui < run.unit_end; ui += kWarps)
                     sweep_unit(q.units[ui], q.rec, op, lane);
@@ -799,6 +807,11 @@ gs_status run_wk_queries(gs_batch* b, std::vector<int>& idx) {
             d.rec = g->d_rec;
             d.R = g->d_runs_blk ? g->R_blk : g->R;
             d.words = N / 32;
+            if (q.algo == GS_ALGO_KCORE && gs_adj_ready(g, 4)) {
+                d.off = g->adj.off_in;
+                d.adj = g->adj.adj_in;
+                d.R = (d.words + kAdjWords - 1) / kAdjWords;
+            }
             d.nw = g->nw;
             d.algo = (int)q.algo;
             d.k = (int)q.arg;

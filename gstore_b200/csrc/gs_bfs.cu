@@ -394,26 +394,34 @@ gs_status gs_graph_nonisolated(gs_graph* g) {
 gs_status bfs_init(gs_state* s) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
+    // every array of the state in one block, cleared by one memset (a small
+    // graph's BFS takes ~100 us in all, a stream operation ~2 of them)
     const uint64_t words = g->N / 32;
-    if (!s->d_depth) GS_TRY(gs_state_alloc(s, (void**)&s->d_depth, g->N));
-    if (!s->d_front) GS_TRY(gs_state_alloc(s, (void**)&s->d_front, words * 8));    // 2-bit state
-    if (!s->d_visited) GS_TRY(gs_state_alloc(s, (void**)&s->d_visited, words * 4)); // next bitmap
-    if (!s->d_act) GS_TRY(gs_state_alloc(s, (void**)&s->d_act, g->nw));
-    if (!s->d_act_next) GS_TRY(gs_state_alloc(s, (void**)&s->d_act_next, g->nw));
-    if (!s->d_error) GS_TRY(gs_state_alloc(s, (void**)&s->d_error, sizeof(uint64_t)));
-    if (!s->d_ticket) GS_TRY(gs_state_alloc(s, (void**)&s->d_ticket, 2 * sizeof(uint32_t)));
     const size_t dead_bytes = ((g->U + 3) & ~(uint64_t)3) + 4;   // whole 32-bit words
-    if (!s->d_dead) GS_TRY(gs_state_alloc(s, (void**)&s->d_dead, dead_bytes));
-    if (!s->d_read) GS_TRY(gs_state_alloc(s, (void**)&s->d_read, 256 * sizeof(unsigned long long)));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_ticket, 0, 2 * sizeof(uint32_t), ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_dead, 0, dead_bytes, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_read, 0, 256 * sizeof(unsigned long long), ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_depth, 0, g->N, ctx->stream));   // INFTY = 0
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_front, 0, words * 8, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_visited, 0, words * 4, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_act, 0, g->nw, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_act_next, 0, g->nw, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_error, 0, sizeof(uint64_t), ctx->stream));
+    size_t total = 0;
+    auto part = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t o_depth = part(g->N), o_front = part(words * 8), o_next = part(words * 4), o_act = part(g->nw),
+                 o_act_next = part(g->nw), o_error = part(sizeof(uint64_t)), o_ticket = part(2 * sizeof(uint32_t)),
+                 o_read = part(256 * sizeof(unsigned long long)), o_ctl = part(kBfsCtlBytes), o_dead = part(dead_bytes);
+    if (!s->d_depth) {
+        uint8_t* p = nullptr;
+        GS_TRY(gs_state_alloc(s, (void**)&p, total));
+        s->d_depth = p + o_depth;
+        s->d_front = (uint32_t*)(p + o_front);     // 2-bit state
+        s->d_visited = (uint32_t*)(p + o_next);    // next bitmap
+        s->d_act = p + o_act;
+        s->d_act_next = p + o_act_next;
+        s->d_error = (uint64_t*)(p + o_error);
+        s->d_ticket = (uint32_t*)(p + o_ticket);
+        s->d_read = (unsigned long long*)(p + o_read);
+        s->d_bfs_ctl = p + o_ctl;
+        s->d_dead = p + o_dead;
+    }
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(s->d_depth, 0, total, ctx->stream));   // INFTY = 0
     bfs_seed_kernel<<<1, 1, 0, ctx->stream>>>(s->d_depth, s->d_front, s->d_act, (uint64_t)s->arg);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
@@ -422,20 +430,12 @@ gs_status bfs_init(gs_state* s) {
     s->level_skip.clear();
     s->level = 1;
     s->level_counts.clear();
-    s->n_act_hist = 0;
     return GS_OK;
 }
 
 gs_status bfs_sweep_begin(gs_state* s) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
-    // Window flags of this sweep, kept on the device for the swept-record
-    // statistics (read back only when asked for: no host round trip here).
-    if (!s->d_act_hist) GS_TRY(gs_state_alloc(s, (void**)&s->d_act_hist, (size_t)g->nw * 256));
-    if (s->n_act_hist < 256)
-        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(s->d_act_hist + (size_t)s->n_act_hist * g->nw, s->d_act, g->nw,
-                                           cudaMemcpyDeviceToDevice, ctx->stream));
-    s->n_act_hist += 1;
     GS_CHECK_CUDA(ctx, (gs_smem_limit_once<bfs_run_kernel<false, false>>(ctx->device, (int)sizeof(BfsSmem))));
     GS_CHECK_CUDA(ctx, (gs_smem_limit_once<bfs_run_kernel<true, false>>(ctx->device, (int)sizeof(BfsSmem))));
     GS_CHECK_CUDA(ctx, (gs_smem_limit_once<bfs_run_kernel<true, true>>(ctx->device, (int)sizeof(BfsSmem))));

@@ -283,6 +283,7 @@ extern "C" gs_status gs_convert(gs_ctx* ctx, const uint32_t* pairs, uint64_t n_p
     gs_dev_free(d_copy);
     if (st != GS_OK) return st;
     st = gs_graph_adopt(ctx, V, d_start, n_start, d_rec, n_rec, d_deg, out);
+    if (st == GS_OK) (*out)->degree_from_records = true;
     gs_dev_free(d_start);
     gs_dev_free(d_deg);
     return st;

@@ -154,6 +154,19 @@ struct gs_rl_layout {
     bool refused = false;            // another layout sweeps this graph faster
 };
 
+// Adjacency lists (gs_adj.cu): the neighbours that a record leads from (in)
+// and to (out); one list on the half grid, whose records lead both ways.
+struct gs_adj {
+    uint32_t *off_in = nullptr, *adj_in = nullptr;     // off: N + 1
+    uint32_t *off_out = nullptr, *adj_out = nullptr;
+    uint32_t* first_in = nullptr;    // N: every vertex's first in-entry
+    uint32_t* none = nullptr;        // N / 32 words: vertices without in-entries
+    uint32_t* hub = nullptr;         // N / 32 words: vertices with over four times the mean entries
+    uint64_t n_in = 0, n_cand = 0;   // in-entries, vertices that have some
+    uint32_t credit = 0;             // sweeps of the grid done by whole queries
+    bool built = false, refused = false;
+};
+
 struct gs_streamer;   // pinned-host record stream of a graph (gs_stream.cu)
 struct gs_seglists;   // double-buffered entry lists of segment sweeps (gs_stream.cu)
 
@@ -186,6 +199,8 @@ struct gs_ctx {
     // the next batch instead of cudaMalloc / cudaFree)
     std::multimap<size_t, void*> pool_free;
     uint64_t pool_bytes = 0;
+    int adj_ctas[2] = {0, 0};        // resident CTAs per SM of the BFS and k-core launches on lists (0: not asked yet)
+    std::vector<struct gs_graph*> adj_graphs;   // graphs with adjacency lists
 };
 
 struct gs_graph {
@@ -221,12 +236,13 @@ struct gs_graph {
     SegView seg;                      // set during segment sweeps
     gs_pr_layout pr;                  // row-slice PageRank layout (serving, batches, smaller graphs)
     gs_pb_layout pb;                  // propagation-blocked PageRank layout (serving, gs_run on large graphs without hubs)
+    gs_adj adj;                       // adjacency lists (gs_run's BFS, WCC and k-core)
     gs_rl_layout rl;                  // row-list PageRank layout (gs_run)
     gs_streamer* stream = nullptr;    // non-null: records stay in host memory
     gs_seglists* lists = nullptr;     // segment entry lists of segment sweeps
     std::vector<gs_tile_run> h_runs;  // host copies of the run and unit tables
     std::vector<gs_unit> h_units;
-    bool degree_from_records = false;
+    bool degree_from_records = false; // d_degree was counted from these records (not the caller's array)
     std::vector<uint64_t> h_start;    // full .start copy (host), for planners
     std::vector<uint64_t> h_tile_off; // host copy of d_tile_off
     std::vector<uint32_t> h_tile_rc;  // host copy of d_tile_rc
@@ -259,7 +275,6 @@ struct gs_state {
     uint8_t* d_act_next = nullptr;   // nw
     std::vector<uint64_t> level_counts;
     uint8_t* d_act_hist = nullptr;   // 256 x nw: each level's window flags (swept-record statistics)
-    int n_act_hist = 0;              // levels recorded in d_act_hist
     // PageRank
     float* d_x = nullptr;            // N
     float* d_y = nullptr;            // N
@@ -272,6 +287,8 @@ struct gs_state {
     // k-core
     int32_t* d_deg = nullptr;        // N
     uint32_t* d_kactive = nullptr;   // N/32
+    void* d_bfs_ctl = nullptr;       // BFS on adjacency lists: control block (kBfsCtlBytes, cleared by bfs_init)
+    void* d_adj = nullptr;           // BFS, k-core on adjacency lists: queues, row chunks (k-core: control block)
     // bfs2 / traverse
     uint32_t* d_lab = nullptr;       // N: depth (bfs2) or colour (traverse)
     int64_t last_count = 0;
@@ -440,6 +457,26 @@ const uint32_t* gs_stream_records(const gs_graph* g);   // host records of a str
 gs_status gs_stream_open_file(gs_graph* g, const char* path, uint64_t segment_bytes);
 // Copies a streamed graph's records (from memory or the file) to dst.
 bool gs_stream_read_records(const gs_graph* g, uint32_t* dst);
+
+// ------------------------------------------------------ adjacency lists --
+// True when whole queries on g run on its adjacency lists.  Counts `sweeps`
+// (what the query costs otherwise, in sweeps of the grid) until kAdjBuild of
+// them have been made, then builds the lists (once, if they fit).
+constexpr uint32_t kAdjBuild = 32;
+constexpr size_t kBfsCtlBytes = 4352;
+bool gs_adj_ready(gs_graph* g, uint32_t sweeps);
+void gs_adj_free(gs_graph* g);
+void gs_adj_release(gs_ctx* ctx);   // drops every graph's lists (an allocation failed)
+// Whole queries from their initial state.  s->done stays false when the lists
+// were dropped meanwhile (nothing has run then).
+gs_status bfs_adj_run(gs_state* s, int64_t* steps);
+gs_status kcore_adj_run(gs_state* s, int64_t* steps);
+// A finished BFS: the windows that held a frontier vertex at levels 1 ..
+// `levels`, from the depths, into s->d_act_hist.
+gs_status gs_level_windows(gs_state* s, int levels);
+// The hooks of a WCC sweep; `vote` launches the choice of the largest tree and
+// its bitmap (s->d_giant) after the first neighbours' hooks.
+gs_status wcc_adj_hook(gs_state* s, void (*vote)(gs_state*), unsigned long long* unresolved);
 
 // bfs2 (-j 30) and traverse (-j 4): one u32 label per vertex in d_lab
 gs_status lab_init(gs_state* s);

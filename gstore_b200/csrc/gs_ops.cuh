@@ -66,6 +66,46 @@ __device__ __forceinline__ void warp_add_u64(unsigned long long* dst, uint64_t v
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(dst, (unsigned long long)v);
 }
 
+// ------------------------------------------------------------ grid barrier --
+constexpr uint64_t kBarrierNs = 4000000000ull;   // 4 s
+
+__device__ __forceinline__ uint64_t global_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Grid-wide barrier of a cooperative launch.  bar[0] counts arrivals, bar[1]
+// is the generation.  False when the wait gave up or another CTA failed.
+__device__ inline bool grid_barrier(unsigned int* bar, int* err) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        volatile unsigned int* vgen = bar + 1;
+        const unsigned int gen = *vgen;
+        __threadfence();
+        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
+            atomicExch(bar, 0u);
+            __threadfence();
+            atomicAdd(bar + 1, 1u);
+        } else {
+            const uint64_t t0 = global_ns();
+            while (*vgen == gen) {
+                if (*(volatile int*)err) break;
+                if (global_ns() - t0 > kBarrierNs) {
+                    atomicOr(err, 1);
+                    break;
+                }
+                __nanosleep(100);
+            }
+        }
+        __threadfence();
+        ok = *(volatile int*)err == 0;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
 // --------------------------------------------------------------- PageRank --
 // Acc: the type of the sums in y.  The sweep of a streamed graph adds in
 // double: its per-record atomics reach high-degree vertices in file order,

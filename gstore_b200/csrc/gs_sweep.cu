@@ -691,10 +691,32 @@ uint32_t gs_wcc_sample_shift(const gs_graph* g) {
     return v <= 0 ? 0u : (uint32_t)std::min<long>(v, 10);
 }
 
+// Launches the vote for the largest tree and, after it, pointer jumping with
+// the tree's bitmap.
+static void wcc_vote(gs_state* s) {
+    gs_graph* g = s->g;
+    gs_ctx* ctx = g->ctx;
+    uint32_t* d_root = s->d_giant + g->N / 32;
+    wcc_giant_root_kernel<<<1, kGiantSamples, 0, ctx->stream>>>(s->d_parent, g->V, d_root);
+    wcc_compress_giant_kernel<<<blocks_for(g->N, ctx), kThreads, 0, ctx->stream>>>(s->d_parent, s->d_giant,
+                                                                                    d_root, g->N);
+    ctx->launches += 2;
+}
+
 gs_status wcc_sweep_launch(gs_state* s) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
     const uint64_t bytes = 4 * g->E + 8 * g->V;
+    if (s->step == 0 && g->adj.built && !g->seg.list) {
+        if (!s->d_giant) GS_TRY(gs_state_alloc(s, (void**)&s->d_giant, (g->N / 32 + 2) * 4));
+        if (g->adj.built) {   // not dropped by that allocation
+            s->wcc_giant = false;
+            gs_timer_begin(ctx);
+            GS_TRY(wcc_adj_hook(s, wcc_vote, (unsigned long long*)ctx->d_scalars));
+            gs_timer_end(ctx, GS_ALGO_WCC, bytes);
+            return GS_OK;
+        }
+    }
     const uint32_t shift = s->step == 0 ? gs_wcc_sample_shift(g) : 0;
     if (shift == 0) {
         // later sweeps (only after a record ran out of hooking retries) keep
@@ -710,7 +732,6 @@ gs_status wcc_sweep_launch(gs_state* s) {
     // then sweep every record, skipping those with both ends in that tree.
     GS_TRY(gs_ensure_blocked(g));
     if (!s->d_giant) GS_TRY(gs_state_alloc(s, (void**)&s->d_giant, (g->N / 32 + 2) * 4));
-    uint32_t* d_root = s->d_giant + g->N / 32;
     // the sampled pass walks the L2-blocked runs (its hooks land on parents
     // of a few windows at a time); the full pass walks the longest-first runs
     // of the BFS sweep (one row window staged per long run), since few of
@@ -727,14 +748,12 @@ gs_status wcc_sweep_launch(gs_state* s) {
     wcc_hook_runs<<<grid, kThreads, 0, ctx->stream>>>(blk ? g->d_runs_blk : g->d_runs, n,
                                                       blk ? g->d_units_blk : g->d_units, g->d_rec, s->d_parent,
                                                       nullptr, nullptr, nullptr, shift, ctx->d_ticket);
-    wcc_giant_root_kernel<<<1, kGiantSamples, 0, ctx->stream>>>(s->d_parent, g->V, d_root);
-    wcc_compress_giant_kernel<<<blocks_for(g->N, ctx), kThreads, 0, ctx->stream>>>(s->d_parent, s->d_giant,
-                                                                                    d_root, g->N);
+    wcc_vote(s);
     wcc_hook_runs<<<grid_full, kThreads, 0, ctx->stream>>>(lpt ? g->d_runs_lpt : g->d_runs, n_full, g->d_units,
                                                            g->d_rec, s->d_parent, s->d_touched, s->d_giant,
                                                            (unsigned long long*)ctx->d_scalars, 0, ctx->d_ticket);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
-    ctx->launches += 4;
+    ctx->launches += 2;
     s->wcc_giant = true;
     gs_timer_end(ctx, GS_ALGO_WCC, bytes);
     return GS_OK;

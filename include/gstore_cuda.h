@@ -200,7 +200,12 @@ gs_status gs_sweep(gs_state* s, const gs_segment* segs, int n_segs);
  * iteration just finished.  done_out: 1 when the algorithm has finished. */
 gs_status gs_finalize(gs_state* s, int64_t* frontier_out, int* done_out);
 /* Sweep + finalize until done, all on the device (one 8-byte read per step).
- * steps_out: number of sweeps. */
+ * steps_out: number of sweeps.  Once whole queries have swept a resident graph
+ * often enough (about eight BFS or k-core queries), and while HBM has room, the
+ * graph also keeps its records as adjacency lists (8 bytes per record and 12
+ * per vertex until gs_graph_free, dropped earlier when an allocation fails), and BFS,
+ * WCC and k-core run on those: the same results and step counts, in one to
+ * eight launches. */
 gs_status gs_run(gs_state* s, int64_t* steps_out);
 
 /* Results.  BFS and BFS2: uint8 depth[V] (root 1, unreached 0, bfs.cpp:54;
@@ -227,7 +232,9 @@ gs_status gs_bfs_stats(gs_state* s, uint64_t* edges_in_component, uint64_t* swep
  * earlier level: such a record can discover nothing, so depths are the
  * same; a streamed graph reads every record of the swept tiles).  Same
  * reference rule otherwise as gs_bfs_stats; no counterpart in the
- * reference, which reads every record of a swept tile. */
+ * reference, which reads every record of a swept tile.  A BFS that gs_run
+ * ran on the graph's adjacency lists reports the list entries it read (4
+ * bytes like a record; on the half grid every record has two). */
 gs_status gs_bfs_records_read(gs_state* s, uint64_t* read_records, int max_levels, int* n_levels);
 
 /* BFS without any allocation (no counterpart in the reference; added for

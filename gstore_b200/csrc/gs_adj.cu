@@ -1066,7 +1066,10 @@ bool gs_adj_ready(gs_graph* g, uint32_t sweeps) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
     if ((keep + g->N * 16 + g->U * 32) * 2 > free_b || g->U >= (1ull << 32)) return false;
-    if (adj_build(g) != GS_OK) return false;   // out of memory after all: the sweeps still run
+    if (adj_build(g) != GS_OK) {
+        A.refused = true;   // out of memory after all: the sweeps still run
+        return false;
+    }
     A.refused = false;
     ctx->adj_graphs.push_back(g);
     return true;

@@ -779,6 +779,8 @@ gs_status run_wk_queries(gs_batch* b, std::vector<int>& idx) {
     gs_ctx* ctx = b->ctx;
     for (size_t s = 0; s < idx.size(); s += kMaxBatch) {
         const size_t e = std::min(idx.size(), s + kMaxBatch);
+        for (size_t k = s; k < e; ++k)
+            if (b->q[idx[k]].algo == GS_ALGO_KCORE) gs_adj_ready(b->q[idx[k]].g, 4);
         std::vector<BQuery> dq;
         for (size_t k = s; k < e; ++k) {
             gs_batch_query& q = b->q[idx[k]];
@@ -807,11 +809,6 @@ gs_status run_wk_queries(gs_batch* b, std::vector<int>& idx) {
             d.rec = g->d_rec;
             d.R = g->d_runs_blk ? g->R_blk : g->R;
             d.words = N / 32;
-            if (q.algo == GS_ALGO_KCORE && gs_adj_ready(g, 4)) {
-                d.off = g->adj.off_in;
-                d.adj = g->adj.adj_in;
-                d.R = (d.words + kAdjWords - 1) / kAdjWords;
-            }
             d.nw = g->nw;
             d.algo = (int)q.algo;
             d.k = (int)q.arg;
@@ -832,7 +829,16 @@ gs_status run_wk_queries(gs_batch* b, std::vector<int>& idx) {
         int* err = (int*)((char*)base + qb + 16);
         unsigned int* tickets = (unsigned int*)((char*)base + qb + 32);   // 4, zeroed with bar and err
         int* sweeps = (int*)((char*)base + qb + 256);
-        for (int k = 0; k < nq; ++k) dq[k].sweeps = sweeps + k;
+        for (int k = 0; k < nq; ++k) {
+            dq[k].sweeps = sweeps + k;
+            // (every buffer is there: an allocation may drop adjacency lists)
+            const gs_adj& A = b->q[idx[s + k]].g->adj;
+            if (dq[k].algo == (int)GS_ALGO_KCORE && A.built) {
+                dq[k].off = A.off_in;
+                dq[k].adj = A.adj_in;
+                dq[k].R = (dq[k].words + kAdjWords - 1) / kAdjWords;
+            }
+        }
         GS_CHECK_CUDA(ctx, cudaMemsetAsync((char*)base + qb, 0, 256 + nq * sizeof(int), ctx->stream));
         GS_CHECK_CUDA(ctx, cudaMemcpyAsync(d_q, dq.data(), nq * sizeof(BQuery), cudaMemcpyHostToDevice, ctx->stream));
         BatchArgs a{d_q, nq, bar, err, tickets};

@@ -268,78 +268,6 @@ static void free_graph_arrays(gs_graph* g) {
     g->d_degree = nullptr;
 }
 
-// An L2-blocked sweep order: tiles grouped into blocks of `block` x `block`
-// windows (row-major inside a block), so the vertex state the tiles in
-// flight touch (2 `block` windows) stays in L2.  Runs are short (one tile
-// row, <= kBlockRunUnits units, one per warp of a CTA) so the CTAs in flight
-// work inside one or two blocks.  Used by the sweeps whose per-record state
-// is large (WCC, k-core, batches, serving: kBlockWindows; multi-source BFS
-// with 16-byte vertex state may pick kBlockWindowsSmall); their results do
-// not depend on the order.
-static gs_status build_blocked_order(gs_graph* g, uint32_t block, uint64_t* R_out, gs_tile_run** d_runs_out,
-                                     gs_unit** d_units_out) {
-    gs_ctx* ctx = g->ctx;
-    const uint64_t T = g->T;
-    std::vector<uint32_t> tile_unit(T + 1, 0);
-    {
-        uint64_t k = 0;
-        for (uint32_t u = 0; u < g->U; ++u) {
-            while (g->h_tile_off[k + 1] <= g->h_units[u].rec_beg) tile_unit[++k] = u;
-        }
-        while (k < T) tile_unit[++k] = (uint32_t)g->U;
-    }
-    std::vector<uint32_t> order(T);
-    for (uint32_t k = 0; k < T; ++k) order[k] = k;
-    auto block_of = [&](uint32_t k) {
-        const uint32_t rc = g->h_tile_rc[k];
-        return ((uint64_t)((rc >> 16) / block) << 32) | ((rc & 0xFFFFu) / block);
-    };
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return block_of(a) < block_of(b); });
-    std::vector<gs_unit> units;
-    std::vector<gs_tile_run> runs;
-    units.reserve(g->U);
-    uint64_t open_block = ~0ull;
-    uint32_t open_row = ~0u;
-    bool is_open = false;
-    for (uint32_t k : order) {
-        const uint32_t row = g->h_tile_rc[k] >> 16;
-        const uint64_t blk = block_of(k);
-        for (uint32_t u = tile_unit[k]; u < tile_unit[k + 1]; ++u) {
-            const gs_unit& d = g->h_units[u];
-            if (!is_open || row != open_row || blk != open_block || runs.back().unit_end - runs.back().unit_beg >= kBlockRunUnits) {
-                runs.push_back(gs_tile_run{d.rec_beg, d.rec_beg, 0, 0, (uint32_t)units.size(), (uint32_t)units.size()});
-                open_row = row;
-                open_block = blk;
-                is_open = true;
-            }
-            units.push_back(d);
-            runs.back().rec_end = d.rec_beg + d.n;
-            runs.back().unit_end = (uint32_t)units.size();
-        }
-    }
-    *R_out = runs.size();
-    GS_TRY(gs_graph_alloc(g, (void**)d_units_out, std::max<size_t>(1, units.size()) * sizeof(gs_unit)));
-    GS_TRY(gs_graph_alloc(g, (void**)d_runs_out, std::max<size_t>(1, runs.size()) * sizeof(gs_tile_run)));
-    if (!units.empty())
-        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(*d_units_out, units.data(), units.size() * sizeof(gs_unit),
-                                           cudaMemcpyHostToDevice, ctx->stream));
-    if (!runs.empty())
-        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(*d_runs_out, runs.data(), runs.size() * sizeof(gs_tile_run),
-                                           cudaMemcpyHostToDevice, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return GS_OK;
-}
-
-// The L2-blocked orders of a resident graph, built at their first use (the
-// BFS sweep and a plain upload do not need them).
-gs_status gs_ensure_blocked(gs_graph* g) {
-    if (g->stream || g->blocked_built) return GS_OK;
-    GS_TRY(build_blocked_order(g, kBlockWindows, &g->R_blk, &g->d_runs_blk, &g->d_units_blk));
-    GS_TRY(build_blocked_order(g, kBlockWindowsSmall, &g->R_blk2, &g->d_runs_blk2, &g->d_units_blk2));
-    g->blocked_built = true;
-    return GS_OK;
-}
-
 // Builds the non-empty tile table and the work items from the host .start
 // array, walking the stored tiles in file order (the loops of grid::*_mmap,
 // gstore.cpp:2520-2559), and uploads them.

@@ -754,8 +754,9 @@ gs_status run_bfs_queries(gs_batch* b, std::vector<int>& idx) {
             if (b->q[i].g == g) mine.push_back(i);
         const int cand = pick_candidate(tune_of(g));
         const int bits = cand >= kOrders ? 64 : 32;
-        GS_TRY(gs_ensure_blocked(g));
-        const int order = g->d_runs_blk ? cand % kOrders : 0;
+        const int order = cand % kOrders;
+        if (order == 1) GS_TRY(gs_ensure_blocked(g));
+        if (order == 2) GS_TRY(gs_ensure_blocked_small(g));
         if (order == 3 && !g->pr.built) GS_TRY(pr_layout_build(g));
         for (size_t s = 0; s < mine.size(); s += bits) {
             gs_bfs_group grp;

@@ -53,8 +53,19 @@ void gs_dev_free(void* ptr) {
 
 constexpr uint64_t kPoolMaxBytes = 16ull << 30;
 
+// Block sizes: multiples of 256 bytes; between 64 KiB and 1 GiB rounded up to
+// 32 steps per power of two (at most 3 % more), so that blocks of nearly equal
+// size -- the records of two graphs of one shape -- serve one another.
+static size_t pool_size(size_t bytes) {
+    size_t step = 256;
+    if (bytes >= (64u << 10) && bytes < (1ull << 30))
+        while (step * 64 <= bytes) step *= 2;
+    return (bytes + step - 1) & ~(step - 1);
+}
+
 gs_status gs_pool_get(gs_ctx* ctx, size_t bytes, void** out) {
-    bytes = (bytes + 255) & ~(size_t)255;
+    *out = nullptr;
+    bytes = pool_size(bytes);
     auto it = ctx->pool_free.find(bytes);
     if (it != ctx->pool_free.end()) {
         *out = it->second;
@@ -67,7 +78,7 @@ gs_status gs_pool_get(gs_ctx* ctx, size_t bytes, void** out) {
 
 void gs_pool_put(gs_ctx* ctx, void* ptr, size_t bytes) {
     if (!ptr) return;
-    bytes = (bytes + 255) & ~(size_t)255;
+    bytes = pool_size(bytes);
     if (ctx->pool_bytes + bytes > kPoolMaxBytes) {
         gs_dev_free(ptr);
         return;
@@ -456,18 +467,20 @@ static gs_status new_graph(gs_ctx* ctx, uint64_t V, gs_graph** out) {
     return GS_OK;
 }
 
-// Builds a resident graph around records already in device memory
-// (d_rec is adopted; d_start and d_degree are copied and stay the caller's).
+// Builds a resident graph around records already in device memory (d_rec, a
+// pool block of n_edges + kRecPad records, is adopted; d_start and d_degree are
+// copied and stay the caller's).
 gs_status gs_graph_adopt(gs_ctx* ctx, uint64_t V, const uint64_t* d_start, uint64_t n_start, uint32_t* d_rec,
                          uint64_t n_edges, const int32_t* d_degree, gs_graph** out) {
     *out = nullptr;
     gs_graph* g = nullptr;
     gs_status st = new_graph(ctx, V, &g);
     if (st != GS_OK) {
-        gs_dev_free(d_rec);
+        gs_pool_put(ctx, d_rec, (n_edges + kRecPad) * 4);
         return st;
     }
     g->d_rec = d_rec;
+    g->pooled.emplace_back((void*)d_rec, (size_t)(n_edges + kRecPad) * 4);
     g->E = n_edges;
     g->h_start.resize(n_start);
     cudaError_t e = cudaMemcpyAsync(g->h_start.data(), d_start, n_start * 8, cudaMemcpyDeviceToHost, ctx->stream);

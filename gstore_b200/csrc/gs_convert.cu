@@ -75,6 +75,79 @@ __global__ void scatter_kernel(const uint2* __restrict__ pairs, uint64_t n, uint
     }
 }
 
+// The same two passes for grids of at most kSmemTiles stored tiles (V <= 2^24):
+// a CTA takes a stretch of the edges and keeps its own tile counters in shared
+// memory.  One counter in global memory per tile means tens of thousands of
+// atomics on the same few addresses, and a slot taken one by one scatters
+// single records: 1.60 and 1.89 ms for the 67 M edges of Kronecker 22 (2,080
+// tiles in use).  Here a tile's counter is added to, and its slots are
+// reserved, once per CTA and stretch, whose records of a tile then lie side by
+// side: 0.94 and 0.98 ms.  What is left of the count are the two
+// random degree atomics per edge (~180 G/s).
+constexpr uint64_t kSmemTiles = 49152;         // 192 KB of counters
+constexpr uint64_t kSmemMinEdges = 1u << 20;   // fewer: clearing and reading the counters costs more than it saves
+constexpr int kSmemThreads = 1024;
+
+__global__ void __launch_bounds__(kSmemThreads, 1)
+    count_smem_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t V, uint64_t p, int directed, uint32_t T,
+                      unsigned long long* __restrict__ counts, int32_t* __restrict__ deg, int* bad) {
+    extern __shared__ uint32_t s_count[];
+    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads) s_count[t] = 0;
+    __syncthreads();
+    const uint64_t nth = (uint64_t)gridDim.x * kSmemThreads;
+    for (uint64_t k = (uint64_t)blockIdx.x * kSmemThreads + threadIdx.x; k < n; k += 4 * nth) {
+        uint2 e[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = k + j * nth < n ? __ldcs(pairs + k + j * nth) : make_uint2(0, 0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (e[j].x == e[j].y) continue;  // is_self_loop
+            if (e[j].x >= V || e[j].y >= V) {
+                *bad = 1;
+                continue;
+            }
+            const bool swap = !directed && e[j].x > e[j].y;
+            const uint64_t a = swap ? e[j].y : e[j].x, b = swap ? e[j].x : e[j].y;
+            atomicAdd(s_count + tile_of(a, b, p, directed), 1u);
+            atomicAdd(deg + e[j].x, 1);
+            if (!directed) atomicAdd(deg + e[j].y, 1);
+        }
+    }
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads)
+        if (s_count[t]) atomicAdd(counts + t, (unsigned long long)s_count[t]);
+}
+
+__global__ void __launch_bounds__(kSmemThreads, 1)
+    scatter_smem_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t per, uint64_t p, int directed, uint32_t T,
+                        const uint64_t* __restrict__ start, unsigned int* __restrict__ cursor,
+                        uint32_t* __restrict__ rec) {
+    extern __shared__ uint32_t s_slot[];
+    const uint64_t lo = (uint64_t)blockIdx.x * per, hi = lo + per < n ? lo + per : n;
+    auto each = [&](auto fn) {
+        for (uint64_t k = lo + threadIdx.x; k < hi; k += 4 * kSmemThreads) {
+            uint2 e[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) e[j] = k + j * kSmemThreads < hi ? pairs[k + j * kSmemThreads] : make_uint2(0, 0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (e[j].x == e[j].y) continue;
+                const bool swap = !directed && e[j].x > e[j].y;
+                const uint64_t a = swap ? e[j].y : e[j].x, b = swap ? e[j].x : e[j].y;
+                fn((uint32_t)tile_of(a, b, p, directed), (uint32_t)(a & 0xFFFF) | ((uint32_t)(b & 0xFFFF) << 16));
+            }
+        }
+    };
+    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads) s_slot[t] = 0;
+    __syncthreads();
+    each([&](uint32_t t, uint32_t) { atomicAdd(s_slot + t, 1u); });
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads)
+        if (const uint32_t c = s_slot[t]) s_slot[t] = atomicAdd(cursor + t, c);
+    __syncthreads();
+    each([&](uint32_t t, uint32_t r) { rec[start[t] + atomicAdd(s_slot + t, 1u)] = r; });
+}
+
 __global__ void rebase_offsets_kernel(const uint64_t* __restrict__ start, uint64_t t0, uint64_t n,
                                       int* __restrict__ out) {
     const uint64_t base = start[t0];
@@ -122,20 +195,20 @@ gs_status gs_order_tiles(gs_graph* g, bool* sorted_now) {
     return GS_OK;
 }
 
-// Sorts the records of every tile in place (segments = tiles of `start`).
-gs_status gs_sort_tiles(gs_ctx* ctx, const uint64_t* d_start, uint64_t n_tiles, uint32_t* d_rec, uint64_t n_rec) {
-    if (n_rec < 2 || n_tiles == 0) return GS_OK;
+// Sorts the records of every tile (segments = tiles of `start`) from d_rec
+// into d_out.
+static gs_status sort_tiles_into(gs_ctx* ctx, const uint64_t* d_start, uint64_t n_tiles, uint32_t* d_rec,
+                                 uint64_t n_rec, uint32_t* d_out) {
     std::vector<uint64_t> h(n_tiles + 1);
     GS_CHECK_CUDA(ctx, cudaMemcpyAsync(h.data(), d_start, (n_tiles + 1) * 8, cudaMemcpyDeviceToHost, ctx->stream));
     GS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // chunks of whole tiles with at most 2^30 records and 2^24 tiles each
     const uint64_t kMaxRec = 1ull << 30, kMaxTiles = 1ull << 24;
-    uint32_t* d_out = nullptr;
     int* d_off = nullptr;
     void* d_tmp = nullptr;
     size_t tmp_bytes = 0;
-    gs_status st = gs_alloc_records(ctx, &d_out, n_rec);
-    if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&d_off, (std::min(n_tiles, kMaxTiles) + 1) * sizeof(int));
+    const size_t off_bytes = (std::min(n_tiles, kMaxTiles) + 1) * sizeof(int);
+    gs_status st = gs_pool_get(ctx, off_bytes, (void**)&d_off);
     uint64_t t0 = 0;
     while (st == GS_OK && t0 < n_tiles) {
         uint64_t t1 = t0;
@@ -152,10 +225,10 @@ gs_status gs_sort_tiles(gs_ctx* ctx, const uint64_t* d_start, uint64_t n_tiles, 
             cudaError_t e = cub::DeviceSegmentedSort::SortKeys(nullptr, need, d_rec + h[t0], d_out + h[t0], (int)nr,
                                                                (int)(t1 - t0), d_off, d_off + 1, ctx->stream);
             if (e == cudaSuccess && need > tmp_bytes) {
-                gs_dev_free(d_tmp);
+                gs_pool_put(ctx, d_tmp, tmp_bytes);
                 d_tmp = nullptr;
                 tmp_bytes = need;
-                st = gs_dev_alloc(ctx, &d_tmp, tmp_bytes);
+                st = gs_pool_get(ctx, tmp_bytes, &d_tmp);
             }
             if (e == cudaSuccess && st == GS_OK)
                 e = cub::DeviceSegmentedSort::SortKeys(d_tmp, need, d_rec + h[t0], d_out + h[t0], (int)nr,
@@ -168,6 +241,18 @@ gs_status gs_sort_tiles(gs_ctx* ctx, const uint64_t* d_start, uint64_t n_tiles, 
         }
         t0 = t1;
     }
+    // (pooled scratch is reused in stream order)
+    gs_pool_put(ctx, d_off, off_bytes);
+    gs_pool_put(ctx, d_tmp, tmp_bytes);
+    return st;
+}
+
+// The same in place.
+gs_status gs_sort_tiles(gs_ctx* ctx, const uint64_t* d_start, uint64_t n_tiles, uint32_t* d_rec, uint64_t n_rec) {
+    if (n_rec < 2 || n_tiles == 0) return GS_OK;
+    uint32_t* d_out = nullptr;
+    GS_TRY(gs_pool_get(ctx, n_rec * 4, (void**)&d_out));
+    gs_status st = sort_tiles_into(ctx, d_start, n_tiles, d_rec, n_rec, d_out);
     if (st == GS_OK) {
         cudaError_t e = cudaMemcpyAsync(d_rec, d_out, n_rec * 4, cudaMemcpyDeviceToDevice, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -175,87 +260,108 @@ gs_status gs_sort_tiles(gs_ctx* ctx, const uint64_t* d_start, uint64_t n_tiles, 
     } else {
         cudaStreamSynchronize(ctx->stream);
     }
-    gs_dev_free(d_out);
-    gs_dev_free(d_off);
-    gs_dev_free(d_tmp);
+    gs_pool_put(ctx, d_out, n_rec * 4);
     return st;
 }
 
-gs_status gs_convert_launch(gs_ctx* ctx, const uint32_t* d_pairs, uint64_t n_pairs, uint64_t V, int directed,
-                            uint64_t** d_start_out, uint32_t** d_grid_out, int32_t** d_degree_out,
-                            uint64_t* n_start, uint64_t* n_rec) {
+
+// Scratch of a conversion goes back to the context's pool (a conversion made
+// seven cudaMalloc / cudaFree pairs, 3 of the 12 ms of Kronecker 22 and up to
+// 0.7 s when the driver is slow), blocks over 1 GiB to the driver.
+static void scratch_put(gs_ctx* ctx, void* p, size_t bytes) {
+    if (bytes > (1ull << 30)) gs_dev_free(p);
+    else gs_pool_put(ctx, p, bytes);
+}
+
+struct gs_converted {
+    uint64_t* d_start = nullptr;
+    int32_t* d_degree = nullptr;
+    uint32_t* d_rec = nullptr;   // n_rec + kRecPad records, the padding zero
+    uint64_t n_start = 0, n_rec = 0, V = 0;
+    size_t rec_bytes() const { return (n_rec + kRecPad) * 4; }
+};
+
+static void converted_put(gs_ctx* ctx, gs_converted& c, bool rec) {
+    scratch_put(ctx, c.d_start, c.n_start * 8);
+    scratch_put(ctx, c.d_degree, std::max<uint64_t>(c.V, 1) * 4);
+    if (rec) scratch_put(ctx, c.d_rec, c.rec_bytes());
+}
+
+static gs_status convert_launch(gs_ctx* ctx, const uint32_t* d_pairs, uint64_t n_pairs, uint64_t V, int directed,
+                                gs_converted& c) {
     uint32_t p, ps;
     uint64_t T;
     gs_geometry_of(V, directed, &p, &ps, &T);
-    uint64_t* d_start = nullptr;
-    unsigned int* d_cursor = nullptr;
-    int32_t* d_deg = nullptr;
-    uint32_t* d_rec = nullptr;
-    void* d_tmp = nullptr;
-    size_t tmp_bytes = 0;
+    cudaStream_t q = ctx->stream;
     int* d_bad = (int*)ctx->d_scalars;
-    gs_status st = GS_OK;
     const uint2* pairs = reinterpret_cast<const uint2*>(d_pairs);
     const uint32_t blocks = (uint32_t)std::max<uint64_t>(
         1, std::min<uint64_t>((n_pairs + 255) / 256, gs_grid_size(ctx, 16)));
-    uint64_t total = 0;
-    int bad = 0;
-#define CV_CHECK(call)                                   \
-    do {                                                 \
-        cudaError_t e_ = (call);                         \
-        if (e_ != cudaSuccess) {                         \
-            st = gs_cuda_fail(ctx, e_, #call);           \
-            goto fail;                                   \
-        }                                                \
-    } while (0)
-    if ((st = gs_dev_alloc(ctx, (void**)&d_start, (T + 1) * 8)) != GS_OK) goto fail;
-    if ((st = gs_dev_alloc(ctx, (void**)&d_deg, std::max<uint64_t>(V, 1) * 4)) != GS_OK) goto fail;
-    CV_CHECK(cudaMemsetAsync(d_start, 0, (T + 1) * 8, ctx->stream));
-    CV_CHECK(cudaMemsetAsync(d_deg, 0, V * 4, ctx->stream));
-    CV_CHECK(cudaMemsetAsync(d_bad, 0, sizeof(int), ctx->stream));
+    const bool smem = T <= kSmemTiles && n_pairs >= kSmemMinEdges;
+    if (smem) {
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<count_smem_kernel>(ctx->device, (int)(kSmemTiles * 4)));
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<scatter_smem_kernel>(ctx->device, (int)(kSmemTiles * 4)));
+    }
+    c.V = V;
+    c.n_start = T + 1;
+    GS_TRY(gs_pool_get(ctx, c.n_start * 8, (void**)&c.d_start));
+    GS_TRY(gs_pool_get(ctx, std::max<uint64_t>(V, 1) * 4, (void**)&c.d_degree));
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_start, 0, c.n_start * 8, q));
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_degree, 0, V * 4, q));
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(d_bad, 0, sizeof(int), q));
+    unsigned long long* counts = (unsigned long long*)c.d_start;
     if (n_pairs) {
-        count_kernel<<<blocks, 256, 0, ctx->stream>>>(pairs, n_pairs, V, p, directed,
-                                                      (unsigned long long*)d_start, d_deg, d_bad);
-        CV_CHECK(cudaGetLastError());
+        if (smem)
+            count_smem_kernel<<<ctx->num_sms, kSmemThreads, T * 4, q>>>(pairs, n_pairs, V, p, directed, (uint32_t)T,
+                                                                        counts, c.d_degree, d_bad);
+        else
+            count_kernel<<<blocks, 256, 0, q>>>(pairs, n_pairs, V, p, directed, counts, c.d_degree, d_bad);
+        GS_CHECK_CUDA(ctx, cudaGetLastError());
         ctx->launches++;
     }
-    CV_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_start, d_start, T + 1, ctx->stream));
-    if ((st = gs_dev_alloc(ctx, &d_tmp, tmp_bytes)) != GS_OK) goto fail;
-    CV_CHECK(cub::DeviceScan::ExclusiveSum(d_tmp, tmp_bytes, d_start, d_start, T + 1, ctx->stream));
-    CV_CHECK(cudaMemcpyAsync(&total, d_start + T, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CV_CHECK(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CV_CHECK(cudaStreamSynchronize(ctx->stream));
-    if (bad) {
-        st = gs_fail(ctx, GS_ERR_FORMAT, "an edge endpoint is >= the vertex count");
-        goto fail;
-    }
-    if ((st = gs_alloc_records(ctx, &d_rec, total)) != GS_OK) goto fail;
-    if ((st = gs_dev_alloc(ctx, (void**)&d_cursor, T * 4)) != GS_OK) goto fail;
-    CV_CHECK(cudaMemsetAsync(d_cursor, 0, T * 4, ctx->stream));
-    if (n_pairs) {
-        scatter_kernel<<<blocks, 256, 0, ctx->stream>>>(pairs, n_pairs, p, directed, d_start, d_cursor, d_rec);
-        CV_CHECK(cudaGetLastError());
-        ctx->launches++;
-    }
-    CV_CHECK(cudaStreamSynchronize(ctx->stream));
-    gs_dev_free(d_cursor);
-    d_cursor = nullptr;
-    if ((st = gs_sort_tiles(ctx, d_start, T, d_rec, total)) != GS_OK) goto fail;
-    gs_dev_free(d_tmp);
-    *d_start_out = d_start;
-    *d_grid_out = d_rec;
-    *d_degree_out = d_deg;
-    *n_start = T + 1;
-    *n_rec = total;
-    return GS_OK;
-fail:
-#undef CV_CHECK
-    cudaStreamSynchronize(ctx->stream);
-    gs_dev_free(d_start);
-    gs_dev_free(d_cursor);
-    gs_dev_free(d_deg);
-    gs_dev_free(d_rec);
-    gs_dev_free(d_tmp);
+    // cub's scratch, then the slot cursors
+    size_t scan_bytes = 0;
+    GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, c.d_start, c.d_start, c.n_start, q));
+    scan_bytes = (scan_bytes + 255) & ~(size_t)255;
+    char* d_tmp = nullptr;
+    const size_t tmp_bytes = scan_bytes + T * 4;
+    GS_TRY(gs_pool_get(ctx, tmp_bytes, (void**)&d_tmp));
+    unsigned int* d_cursor = (unsigned int*)(d_tmp + scan_bytes);
+    gs_status st = [&]() -> gs_status {
+        GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(d_tmp, scan_bytes, c.d_start, c.d_start, c.n_start, q));
+        GS_CHECK_CUDA(ctx, cudaMemsetAsync(d_cursor, 0, T * 4, q));
+        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars, c.d_start + T, 8, cudaMemcpyDeviceToHost, q));
+        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 1, d_bad, sizeof(int), cudaMemcpyDeviceToHost, q));
+        GS_CHECK_CUDA(ctx, cudaStreamSynchronize(q));
+        if (*(const int*)(ctx->h_scalars + 1))
+            return gs_fail(ctx, GS_ERR_FORMAT, "an edge endpoint is >= the vertex count");
+        c.n_rec = ctx->h_scalars[0];
+        GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&c.d_rec));
+        uint32_t* d_raw = nullptr;   // the records before the sort
+        GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&d_raw));
+        const gs_status sorted = [&]() -> gs_status {
+            if (n_pairs) {
+                if (smem) {
+                    const uint64_t per = std::max<uint64_t>(1 << 16, (n_pairs + 2 * ctx->num_sms - 1) / (2 * ctx->num_sms));
+                    scatter_smem_kernel<<<(uint32_t)((n_pairs + per - 1) / per), kSmemThreads, T * 4, q>>>(
+                        pairs, n_pairs, per, p, directed, (uint32_t)T, c.d_start, d_cursor, d_raw);
+                } else {
+                    scatter_kernel<<<blocks, 256, 0, q>>>(pairs, n_pairs, p, directed, c.d_start, d_cursor, d_raw);
+                }
+                GS_CHECK_CUDA(ctx, cudaGetLastError());
+                ctx->launches++;
+            }
+            if (c.n_rec < 2)
+                GS_CHECK_CUDA(ctx, cudaMemcpyAsync(c.d_rec, d_raw, c.n_rec * 4, cudaMemcpyDeviceToDevice, q));
+            else
+                GS_TRY(sort_tiles_into(ctx, c.d_start, T, d_raw, c.n_rec, c.d_rec));
+            GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_rec + c.n_rec, 0, kRecPad * 4, q));
+            return GS_OK;
+        }();
+        scratch_put(ctx, d_raw, c.rec_bytes());
+        return sorted;
+    }();
+    scratch_put(ctx, d_tmp, tmp_bytes);
     return st;
 }
 
@@ -266,25 +372,23 @@ extern "C" gs_status gs_convert(gs_ctx* ctx, const uint32_t* pairs, uint64_t n_p
     const uint32_t* d_pairs = pairs;
     uint32_t* d_copy = nullptr;
     if (!is_device && n_pairs) {
-        GS_TRY(gs_dev_alloc(ctx, (void**)&d_copy, n_pairs * 8));
+        GS_TRY(gs_pool_get(ctx, n_pairs * 8, (void**)&d_copy));
         cudaError_t e = cudaMemcpyAsync(d_copy, pairs, n_pairs * 8, cudaMemcpyHostToDevice, ctx->stream);
         if (e != cudaSuccess) {
-            gs_dev_free(d_copy);
+            scratch_put(ctx, d_copy, n_pairs * 8);
             return gs_cuda_fail(ctx, e, "copy pairs");
         }
         d_pairs = d_copy;
     }
-    uint64_t* d_start = nullptr;
-    uint32_t* d_rec = nullptr;
-    int32_t* d_deg = nullptr;
-    uint64_t n_start = 0, n_rec = 0;
-    gs_status st = gs_convert_launch(ctx, d_pairs, n_pairs, V, ctx->directed, &d_start, &d_rec, &d_deg,
-                                     &n_start, &n_rec);
-    gs_dev_free(d_copy);
-    if (st != GS_OK) return st;
-    st = gs_graph_adopt(ctx, V, d_start, n_start, d_rec, n_rec, d_deg, out);
+    gs_converted c;
+    gs_status st = convert_launch(ctx, d_pairs, n_pairs, V, ctx->directed, c);
+    if (d_copy) scratch_put(ctx, d_copy, n_pairs * 8);
+    if (st != GS_OK) {
+        converted_put(ctx, c, true);
+        return st;
+    }
+    st = gs_graph_adopt(ctx, V, c.d_start, c.n_start, c.d_rec, c.n_rec, c.d_degree, out);
     if (st == GS_OK) (*out)->degree_from_records = true;
-    gs_dev_free(d_start);
-    gs_dev_free(d_deg);
+    converted_put(ctx, c, false);
     return st;
 }

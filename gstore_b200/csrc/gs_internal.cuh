@@ -494,10 +494,6 @@ gs_status gs_swept_records(gs_state* s, const uint8_t* h_act, uint64_t* swept);
 
 gs_status gs_kron_gen_launch(gs_ctx* ctx, int scale, int64_t ef, uint64_t s1, uint64_t s2,
                              uint32_t* d_pairs);
-gs_status gs_convert_launch(gs_ctx* ctx, const uint32_t* d_pairs, uint64_t n_pairs, uint64_t V,
-                            int directed, uint64_t** d_start_out, uint32_t** d_grid_out,
-                            int32_t** d_degree_out, uint64_t* n_start, uint64_t* n_rec);
-
 gs_status gs_sort_tiles(gs_ctx* ctx, const uint64_t* d_start, uint64_t n_tiles, uint32_t* d_rec, uint64_t n_rec);
 // A resident graph whose tiles hold their records out of ascending order
 // (the reference converter leaves them in its threads' order) gets every

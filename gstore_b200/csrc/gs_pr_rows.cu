@@ -34,7 +34,7 @@
 //
 // Per iteration against propagation blocking (gs_pr_blocked.cu: 12.5 bytes
 // moved per entry, a shared-memory atomic per run of destinations): Kronecker
-// 20 / 24 / 26, edge factor 16: 85 / 1,080 / 5,910 us against 146 / 1,862 /
+// 20 / 24 / 26, edge factor 16: 81 / 1,045 / 5,900 us against 146 / 1,862 /
 // 8,010; the layout keeps 4.4 bytes per entry instead of 12.5.  Without hubs
 // (uniform random, 3 M vertices, 24 M entries) 153 against 130: rl_worth.
 // At Kronecker 23 the pull reads 28 % of its entries' sources through L2 and
@@ -754,9 +754,12 @@ gs_status build(gs_graph* g, bool* worth) {
         // the shared-memory pipe busy: both kinds are in flight all the time
         // when the three groups' units take turns
         if (p == 0) interleave(units, G);
-        // clocks of an SM's load path per entry: ~1 from L2, ~0.13 from shared memory
+        // time per entry: 1 from L2, 0.5 from shared memory.  (The load path's
+        // clocks are 1 and 0.13, but what the panels' CTAs run into is latency:
+        // with 0.13 they finished last, 265 against 240 us per iteration at
+        // Kronecker 22, 1,070 against 1,045 at 24; 0.8 and 1.5 are no better.)
         const double cold = p ? 0.0 : (double)(n_ent - hot - std::min<uint64_t>(in_panels, n_ent - hot));
-        cost[p] = cold + 0.13 * ((double)(at_step - step0) * 128 - cold);
+        cost[p] = cold + 0.5 * ((double)(at_step - step0) * 128 - cold);
     }
     L.unit_beg[n_panels] = (uint32_t)units.size();
     L.n_panels = n_panels;

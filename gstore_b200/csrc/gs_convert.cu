@@ -75,27 +75,53 @@ __global__ void scatter_kernel(const uint2* __restrict__ pairs, uint64_t n, uint
     }
 }
 
-// The same two passes for grids of at most kSmemTiles stored tiles (V <= 2^24):
-// a CTA takes a stretch of the edges and keeps its own tile counters in shared
-// memory.  One counter in global memory per tile means tens of thousands of
-// atomics on the same few addresses, and a slot taken one by one scatters
-// single records: 1.60 and 1.89 ms for the 67 M edges of Kronecker 22 (2,080
-// tiles in use).  Here a tile's counter is added to, and its slots are
-// reserved, once per CTA and stretch, whose records of a tile then lie side by
-// side: 0.94 and 0.98 ms.  What is left of the count are the two
-// random degree atomics per edge (~180 G/s).
-constexpr uint64_t kSmemTiles = 49152;         // 192 KB of counters
-constexpr uint64_t kSmemMinEdges = 1u << 20;   // fewer: clearing and reading the counters costs more than it saves
-constexpr int kSmemThreads = 1024;
+// The conversion of graphs of one tile group (V <= 2^24): the edges are split
+// into buckets -- a tile, or 2^bits slices of a tile by the high bits of v1 --
+// whose counters fit one CTA's shared memory, and the buckets are sorted.
+// Buckets in order are tiles in file order, and a tile's sorted slices in order
+// are the sorted tile.
+//   * Counters in global memory, one per tile, take tens of thousands of
+//     atomics on the same few addresses, and slots taken one by one scatter
+//     single records.  Here a CTA takes a stretch of the edges, counts it in
+//     shared memory and reserves each bucket's slots once, so that its records
+//     of a bucket lie side by side.
+//   * A segmented sort gives a segment to a CTA, which needs four passes over
+//     memory for one that does not fit its shared memory: 1.7 ms for the three
+//     tiles of 0.8 M edges over 100,003 vertices.  Slices are small (about
+//     1,024 records and more) and many.
+//   * But not for their own sake: the 2,080 tiles of Kronecker 22 cut into
+//     33,280 slices took 1.82 ms to scatter (shorter stretches) and 2.50 to
+//     sort instead of 0.98 and 2.13.
+// 67 M edges of Kronecker 22, ms: count 1.60 -> 0.94, scatter 1.89 -> 0.98, sort
+// 2.14 as before; 0.8 M edges over 100,003 vertices, all of it: 2.67 -> 0.48.  What
+// is left of the count are the two random degree atomics per edge (~180 G/s).
+constexpr uint32_t kMaxBuckets = 49152;        // 192 KB of counters
+constexpr uint64_t kEnoughBuckets = 2048;      // no more slices from here on (at most 2^12 of one tile)
+constexpr uint64_t kBucketRecords = 1024;      // records a slice should have on average
+constexpr uint64_t kBucketMinEdges = 1u << 14; // fewer: the counters' clearing and reading costs more than it saves
+constexpr int kBucketThreads = 1024;
 
-__global__ void __launch_bounds__(kSmemThreads, 1)
-    count_smem_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t V, uint64_t p, int directed, uint32_t T,
-                      unsigned long long* __restrict__ counts, int32_t* __restrict__ deg, int* bad) {
+struct Buckets {
+    uint32_t nw;     // tiles per side that hold vertices
+    int directed, bits;
+    uint32_t n;      // buckets
+};
+
+__host__ __device__ __forceinline__ uint32_t bucket_tile(uint32_t i, uint32_t j, const Buckets& B) {
+    return B.directed ? i * B.nw + j : i * (2 * B.nw - i + 1) / 2 + (j - i);   // file order
+}
+__device__ __forceinline__ uint32_t bucket_of(uint32_t a, uint32_t b, const Buckets& B) {
+    return (bucket_tile(a >> kTileBits, b >> kTileBits, B) << B.bits) | ((b & 0xFFFFu) >> (kTileBits - B.bits));
+}
+
+__global__ void __launch_bounds__(kBucketThreads, 1)
+    bucket_count_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t V, const Buckets B,
+                        uint32_t* __restrict__ counts, int32_t* __restrict__ deg, int* bad) {
     extern __shared__ uint32_t s_count[];
-    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads) s_count[t] = 0;
+    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads) s_count[t] = 0;
     __syncthreads();
-    const uint64_t nth = (uint64_t)gridDim.x * kSmemThreads;
-    for (uint64_t k = (uint64_t)blockIdx.x * kSmemThreads + threadIdx.x; k < n; k += 4 * nth) {
+    const uint64_t nth = (uint64_t)gridDim.x * kBucketThreads;
+    for (uint64_t k = (uint64_t)blockIdx.x * kBucketThreads + threadIdx.x; k < n; k += 4 * nth) {
         uint2 e[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) e[j] = k + j * nth < n ? __ldcs(pairs + k + j * nth) : make_uint2(0, 0);
@@ -106,46 +132,62 @@ __global__ void __launch_bounds__(kSmemThreads, 1)
                 *bad = 1;
                 continue;
             }
-            const bool swap = !directed && e[j].x > e[j].y;
-            const uint64_t a = swap ? e[j].y : e[j].x, b = swap ? e[j].x : e[j].y;
-            atomicAdd(s_count + tile_of(a, b, p, directed), 1u);
+            const bool swap = !B.directed && e[j].x > e[j].y;
+            atomicAdd(s_count + bucket_of(swap ? e[j].y : e[j].x, swap ? e[j].x : e[j].y, B), 1u);
             atomicAdd(deg + e[j].x, 1);
-            if (!directed) atomicAdd(deg + e[j].y, 1);
+            if (!B.directed) atomicAdd(deg + e[j].y, 1);
         }
     }
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads)
-        if (s_count[t]) atomicAdd(counts + t, (unsigned long long)s_count[t]);
+    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads)
+        if (s_count[t]) atomicAdd(counts + t, s_count[t]);
 }
 
-__global__ void __launch_bounds__(kSmemThreads, 1)
-    scatter_smem_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t per, uint64_t p, int directed, uint32_t T,
-                        const uint64_t* __restrict__ start, unsigned int* __restrict__ cursor,
-                        uint32_t* __restrict__ rec) {
+// cursor: the buckets' starts; on return their ends.
+__global__ void __launch_bounds__(kBucketThreads, 1)
+    bucket_scatter_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t per, const Buckets B,
+                          uint32_t* __restrict__ cursor, uint32_t* __restrict__ rec) {
     extern __shared__ uint32_t s_slot[];
     const uint64_t lo = (uint64_t)blockIdx.x * per, hi = lo + per < n ? lo + per : n;
     auto each = [&](auto fn) {
-        for (uint64_t k = lo + threadIdx.x; k < hi; k += 4 * kSmemThreads) {
+        for (uint64_t k = lo + threadIdx.x; k < hi; k += 4 * kBucketThreads) {
             uint2 e[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) e[j] = k + j * kSmemThreads < hi ? pairs[k + j * kSmemThreads] : make_uint2(0, 0);
+            for (int j = 0; j < 4; ++j) e[j] = k + j * kBucketThreads < hi ? pairs[k + j * kBucketThreads] : make_uint2(0, 0);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (e[j].x == e[j].y) continue;
-                const bool swap = !directed && e[j].x > e[j].y;
-                const uint64_t a = swap ? e[j].y : e[j].x, b = swap ? e[j].x : e[j].y;
-                fn((uint32_t)tile_of(a, b, p, directed), (uint32_t)(a & 0xFFFF) | ((uint32_t)(b & 0xFFFF) << 16));
+                const bool swap = !B.directed && e[j].x > e[j].y;
+                const uint32_t a = swap ? e[j].y : e[j].x, b = swap ? e[j].x : e[j].y;
+                fn(bucket_of(a, b, B), (a & 0xFFFFu) | (b << 16));
             }
         }
     };
-    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads) s_slot[t] = 0;
+    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads) s_slot[t] = 0;
     __syncthreads();
     each([&](uint32_t t, uint32_t) { atomicAdd(s_slot + t, 1u); });
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < T; t += kSmemThreads)
+    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads)
         if (const uint32_t c = s_slot[t]) s_slot[t] = atomicAdd(cursor + t, c);
     __syncthreads();
-    each([&](uint32_t t, uint32_t r) { rec[start[t] + atomicAdd(s_slot + t, 1u)] = r; });
+    each([&](uint32_t t, uint32_t r) { rec[atomicAdd(s_slot + t, 1u)] = r; });
+}
+
+// .start of the one group's 256 x 256 tiles from the buckets' starts
+// (start[n] = total); tiles beyond the vertices are empty.
+__global__ void bucket_start_kernel(const uint32_t* __restrict__ bucket_start, const Buckets B, uint64_t T,
+                                    uint64_t* __restrict__ start) {
+    const uint32_t nth = gridDim.x * blockDim.x;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < kGroupTiles * kGroupTiles; k += nth) {
+        const uint32_t i = k / kGroupTiles, j = k % kGroupTiles;
+        if (k == 0) start[T] = bucket_start[B.n];
+        if (!B.directed && j < i) continue;
+        const uint64_t t = B.directed ? k : dev_calc_index_half(i, j, kGroupTiles);
+        uint32_t at = B.n;
+        if (i < B.nw && j < B.nw) at = bucket_tile(i, j, B) << B.bits;
+        else if (i + 1 < B.nw) at = bucket_tile(i + 1, B.directed ? 0 : i + 1, B) << B.bits;   // the next row
+        start[t] = bucket_start[at];
+    }
 }
 
 __global__ void rebase_offsets_kernel(const uint64_t* __restrict__ start, uint64_t t0, uint64_t n,
@@ -287,6 +329,88 @@ static void converted_put(gs_ctx* ctx, gs_converted& c, bool rec) {
     if (rec) scratch_put(ctx, c.d_rec, c.rec_bytes());
 }
 
+// The two ways to fill c.d_start and c.d_rec; c.d_degree and *d_bad are zero,
+// the count pass has been launched.
+static gs_status fill_buckets(gs_ctx* ctx, const uint2* pairs, uint64_t n_pairs, const Buckets& B, uint32_t* d_bucket,
+                              const int* d_bad, gs_converted& c) {
+    cudaStream_t q = ctx->stream;
+    uint32_t* d_cursor = d_bucket + B.n + 1;
+    size_t scan_bytes = 0, sort_bytes = 0;
+    GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_bucket, d_bucket, B.n + 1, q));
+    char* d_tmp = nullptr;
+    GS_TRY(gs_pool_get(ctx, scan_bytes, (void**)&d_tmp));
+    cudaError_t e = cub::DeviceScan::ExclusiveSum(d_tmp, scan_bytes, d_bucket, d_bucket, B.n + 1, q);
+    scratch_put(ctx, d_tmp, scan_bytes);
+    GS_CHECK_CUDA(ctx, e);
+    GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars, d_bucket + B.n, 4, cudaMemcpyDeviceToHost, q));
+    GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 1, d_bad, sizeof(int), cudaMemcpyDeviceToHost, q));
+    GS_CHECK_CUDA(ctx, cudaMemcpyAsync(d_cursor, d_bucket, (size_t)B.n * 4, cudaMemcpyDeviceToDevice, q));
+    bucket_start_kernel<<<64, 256, 0, q>>>(d_bucket, B, c.n_start - 1, c.d_start);
+    GS_CHECK_CUDA(ctx, cudaGetLastError());
+    GS_CHECK_CUDA(ctx, cudaStreamSynchronize(q));
+    if (*(const int*)(ctx->h_scalars + 1))
+        return gs_fail(ctx, GS_ERR_FORMAT, "an edge endpoint is >= the vertex count");
+    c.n_rec = *(const uint32_t*)ctx->h_scalars;
+    GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&c.d_rec));
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_rec + c.n_rec, 0, kRecPad * 4, q));
+    if (c.n_rec == 0) return GS_OK;
+    uint32_t* d_raw = nullptr;   // the records before the sort
+    GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&d_raw));
+    const uint64_t per = std::max<uint64_t>(4 * kBucketThreads, (n_pairs + 2 * ctx->num_sms - 1) / (2 * ctx->num_sms));
+    bucket_scatter_kernel<<<(uint32_t)((n_pairs + per - 1) / per), kBucketThreads, (size_t)B.n * 4, q>>>(
+        pairs, n_pairs, per, B, d_cursor, d_raw);
+    e = cudaGetLastError();
+    const int* seg = (const int*)d_bucket;   // n_rec <= 2^30
+    if (e == cudaSuccess)
+        e = cub::DeviceSegmentedSort::SortKeys(nullptr, sort_bytes, d_raw, c.d_rec, (int)c.n_rec, (int)B.n, seg, seg + 1, q);
+    gs_status st = e == cudaSuccess ? gs_pool_get(ctx, sort_bytes, (void**)&d_tmp) : GS_OK;
+    if (e == cudaSuccess && st == GS_OK) {
+        e = cub::DeviceSegmentedSort::SortKeys(d_tmp, sort_bytes, d_raw, c.d_rec, (int)c.n_rec, (int)B.n, seg, seg + 1, q);
+        scratch_put(ctx, d_tmp, sort_bytes);
+    }
+    ctx->launches += 4;
+    scratch_put(ctx, d_raw, c.rec_bytes());
+    return e == cudaSuccess ? st : gs_cuda_fail(ctx, e, "converter");
+}
+
+static gs_status fill_tiles(gs_ctx* ctx, const uint2* pairs, uint64_t n_pairs, uint64_t p, int directed,
+                            uint32_t blocks, const int* d_bad, gs_converted& c) {
+    cudaStream_t q = ctx->stream;
+    const uint64_t T = c.n_start - 1;
+    // cub's scratch, then the slot cursors
+    size_t scan_bytes = 0;
+    GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, c.d_start, c.d_start, c.n_start, q));
+    const size_t cursor_at = (scan_bytes + 255) & ~(size_t)255, tmp_bytes = cursor_at + T * 4;
+    char* d_tmp = nullptr;
+    GS_TRY(gs_pool_get(ctx, tmp_bytes, (void**)&d_tmp));
+    unsigned int* d_cursor = (unsigned int*)(d_tmp + cursor_at);
+    const gs_status st = [&]() -> gs_status {
+        GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(d_tmp, scan_bytes, c.d_start, c.d_start, c.n_start, q));
+        GS_CHECK_CUDA(ctx, cudaMemsetAsync(d_cursor, 0, T * 4, q));
+        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars, c.d_start + T, 8, cudaMemcpyDeviceToHost, q));
+        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 1, d_bad, sizeof(int), cudaMemcpyDeviceToHost, q));
+        GS_CHECK_CUDA(ctx, cudaStreamSynchronize(q));
+        if (*(const int*)(ctx->h_scalars + 1))
+            return gs_fail(ctx, GS_ERR_FORMAT, "an edge endpoint is >= the vertex count");
+        c.n_rec = ctx->h_scalars[0];
+        GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&c.d_rec));
+        GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_rec + c.n_rec, 0, kRecPad * 4, q));
+        if (c.n_rec == 0) return GS_OK;
+        uint32_t* d_raw = nullptr;   // the records before the sort
+        GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&d_raw));
+        scatter_kernel<<<blocks, 256, 0, q>>>(pairs, n_pairs, p, directed, c.d_start, d_cursor, d_raw);
+        cudaError_t e = cudaGetLastError();
+        ctx->launches++;
+        gs_status sorted = GS_OK;
+        if (e == cudaSuccess && c.n_rec == 1) e = cudaMemcpyAsync(c.d_rec, d_raw, 4, cudaMemcpyDeviceToDevice, q);
+        else if (e == cudaSuccess) sorted = sort_tiles_into(ctx, c.d_start, T, d_raw, c.n_rec, c.d_rec);
+        scratch_put(ctx, d_raw, c.rec_bytes());
+        return e == cudaSuccess ? sorted : gs_cuda_fail(ctx, e, "converter");
+    }();
+    scratch_put(ctx, d_tmp, tmp_bytes);
+    return st;
+}
+
 static gs_status convert_launch(gs_ctx* ctx, const uint32_t* d_pairs, uint64_t n_pairs, uint64_t V, int directed,
                                 gs_converted& c) {
     uint32_t p, ps;
@@ -297,72 +421,46 @@ static gs_status convert_launch(gs_ctx* ctx, const uint32_t* d_pairs, uint64_t n
     const uint2* pairs = reinterpret_cast<const uint2*>(d_pairs);
     const uint32_t blocks = (uint32_t)std::max<uint64_t>(
         1, std::min<uint64_t>((n_pairs + 255) / 256, gs_grid_size(ctx, 16)));
-    const bool smem = T <= kSmemTiles && n_pairs >= kSmemMinEdges;
-    if (smem) {
-        GS_CHECK_CUDA(ctx, gs_smem_limit_once<count_smem_kernel>(ctx->device, (int)(kSmemTiles * 4)));
-        GS_CHECK_CUDA(ctx, gs_smem_limit_once<scatter_smem_kernel>(ctx->device, (int)(kSmemTiles * 4)));
-    }
     c.V = V;
     c.n_start = T + 1;
     GS_TRY(gs_pool_get(ctx, c.n_start * 8, (void**)&c.d_start));
     GS_TRY(gs_pool_get(ctx, std::max<uint64_t>(V, 1) * 4, (void**)&c.d_degree));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_start, 0, c.n_start * 8, q));
     GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_degree, 0, V * 4, q));
     GS_CHECK_CUDA(ctx, cudaMemsetAsync(d_bad, 0, sizeof(int), q));
-    unsigned long long* counts = (unsigned long long*)c.d_start;
+    // buckets: the tiles that hold vertices, sliced while a slice keeps
+    // kBucketRecords records and the counters fit
+    Buckets B{(uint32_t)((V + 0xFFFF) >> kTileBits), directed, 0, 0};
+    const uint64_t tiles = directed ? (uint64_t)B.nw * B.nw : (uint64_t)B.nw * (B.nw + 1) / 2;
+    if (p == 1 && tiles <= kMaxBuckets && n_pairs >= kBucketMinEdges && n_pairs <= (1ull << 30)) {
+        while (tiles << B.bits < kEnoughBuckets && n_pairs >> (B.bits + 1) >= tiles * kBucketRecords) ++B.bits;
+        B.n = (uint32_t)(tiles << B.bits);
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_count_kernel>(ctx->device, (int)(kMaxBuckets * 4)));
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_scatter_kernel>(ctx->device, (int)(kMaxBuckets * 4)));
+        const size_t bucket_bytes = ((size_t)B.n * 2 + 1) * 4;   // starts, cursors
+        uint32_t* d_bucket = nullptr;
+        GS_TRY(gs_pool_get(ctx, bucket_bytes, (void**)&d_bucket));
+        cudaError_t e = cudaMemsetAsync(d_bucket, 0, ((size_t)B.n + 1) * 4, q);
+        if (e == cudaSuccess) {
+            const uint32_t grid = (uint32_t)std::min<uint64_t>((n_pairs + 4 * kBucketThreads - 1) / (4 * kBucketThreads),
+                                                               gs_grid_size(ctx, 1));
+            bucket_count_kernel<<<grid, kBucketThreads, (size_t)B.n * 4, q>>>(pairs, n_pairs, V, B, d_bucket, c.d_degree,
+                                                                              d_bad);
+            ctx->launches++;
+            e = cudaGetLastError();
+        }
+        const gs_status st = e == cudaSuccess ? fill_buckets(ctx, pairs, n_pairs, B, d_bucket, d_bad, c)
+                                              : gs_cuda_fail(ctx, e, "converter");
+        scratch_put(ctx, d_bucket, bucket_bytes);
+        return st;
+    }
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_start, 0, c.n_start * 8, q));
     if (n_pairs) {
-        if (smem)
-            count_smem_kernel<<<ctx->num_sms, kSmemThreads, T * 4, q>>>(pairs, n_pairs, V, p, directed, (uint32_t)T,
-                                                                        counts, c.d_degree, d_bad);
-        else
-            count_kernel<<<blocks, 256, 0, q>>>(pairs, n_pairs, V, p, directed, counts, c.d_degree, d_bad);
+        count_kernel<<<blocks, 256, 0, q>>>(pairs, n_pairs, V, p, directed, (unsigned long long*)c.d_start, c.d_degree,
+                                            d_bad);
         GS_CHECK_CUDA(ctx, cudaGetLastError());
         ctx->launches++;
     }
-    // cub's scratch, then the slot cursors
-    size_t scan_bytes = 0;
-    GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, c.d_start, c.d_start, c.n_start, q));
-    scan_bytes = (scan_bytes + 255) & ~(size_t)255;
-    char* d_tmp = nullptr;
-    const size_t tmp_bytes = scan_bytes + T * 4;
-    GS_TRY(gs_pool_get(ctx, tmp_bytes, (void**)&d_tmp));
-    unsigned int* d_cursor = (unsigned int*)(d_tmp + scan_bytes);
-    gs_status st = [&]() -> gs_status {
-        GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(d_tmp, scan_bytes, c.d_start, c.d_start, c.n_start, q));
-        GS_CHECK_CUDA(ctx, cudaMemsetAsync(d_cursor, 0, T * 4, q));
-        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars, c.d_start + T, 8, cudaMemcpyDeviceToHost, q));
-        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 1, d_bad, sizeof(int), cudaMemcpyDeviceToHost, q));
-        GS_CHECK_CUDA(ctx, cudaStreamSynchronize(q));
-        if (*(const int*)(ctx->h_scalars + 1))
-            return gs_fail(ctx, GS_ERR_FORMAT, "an edge endpoint is >= the vertex count");
-        c.n_rec = ctx->h_scalars[0];
-        GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&c.d_rec));
-        uint32_t* d_raw = nullptr;   // the records before the sort
-        GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&d_raw));
-        const gs_status sorted = [&]() -> gs_status {
-            if (n_pairs) {
-                if (smem) {
-                    const uint64_t per = std::max<uint64_t>(1 << 16, (n_pairs + 2 * ctx->num_sms - 1) / (2 * ctx->num_sms));
-                    scatter_smem_kernel<<<(uint32_t)((n_pairs + per - 1) / per), kSmemThreads, T * 4, q>>>(
-                        pairs, n_pairs, per, p, directed, (uint32_t)T, c.d_start, d_cursor, d_raw);
-                } else {
-                    scatter_kernel<<<blocks, 256, 0, q>>>(pairs, n_pairs, p, directed, c.d_start, d_cursor, d_raw);
-                }
-                GS_CHECK_CUDA(ctx, cudaGetLastError());
-                ctx->launches++;
-            }
-            if (c.n_rec < 2)
-                GS_CHECK_CUDA(ctx, cudaMemcpyAsync(c.d_rec, d_raw, c.n_rec * 4, cudaMemcpyDeviceToDevice, q));
-            else
-                GS_TRY(sort_tiles_into(ctx, c.d_start, T, d_raw, c.n_rec, c.d_rec));
-            GS_CHECK_CUDA(ctx, cudaMemsetAsync(c.d_rec + c.n_rec, 0, kRecPad * 4, q));
-            return GS_OK;
-        }();
-        scratch_put(ctx, d_raw, c.rec_bytes());
-        return sorted;
-    }();
-    scratch_put(ctx, d_tmp, tmp_bytes);
-    return st;
+    return fill_tiles(ctx, pairs, n_pairs, p, directed, blocks, d_bad, c);
 }
 
 extern "C" gs_status gs_convert(gs_ctx* ctx, const uint32_t* pairs, uint64_t n_pairs, int is_device,

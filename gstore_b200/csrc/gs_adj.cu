@@ -14,13 +14,13 @@
 // the sweeps (the same level sets, component minima and synchronous rounds).
 //
 // Device time per query, tile sweeps against lists: BFS at Kronecker 26 6.35
-// -> 0.55 ms, WCC at 25 2.9 -> 1.5, k-core(8) at 25 3.4 -> 0.70 (edge factor
+// -> 0.55 ms, WCC at 25 2.9 -> 0.68, k-core(8) at 25 3.4 -> 0.70 (edge factor
 // 16).  What bounds them is random 4-byte accesses to L2 (about one per vertex
 // looked at) and the latency of their chains, so every kernel keeps four
 // independent ones per lane in flight and works on compacted lists of the
 // vertices concerned instead of on words with a few bits set.
 //
-// The lists cost 8 bytes per record and 12 per vertex of HBM, and building
+// The lists cost 8 bytes per record and 11 per vertex of HBM, and building
 // them takes about 7 such queries' time (45 ms at Kronecker 26, 22 at 25).  So a
 // graph gets them once its queries have swept it kAdjBuild times, eight BFS or
 // k-core queries or eleven WCC (gs_adj_ready: a graph that is queried only a
@@ -134,12 +134,20 @@ __global__ void adj_none_kernel(const uint32_t* __restrict__ in, uint64_t N, uin
     warp_add_u64(some, local);
 }
 
-__global__ void adj_hub_kernel(const uint32_t* __restrict__ out, uint64_t N, uint32_t least, uint32_t* __restrict__ hub) {
+// The vertices of at least `least` out-entries: their bits, and their list (any
+// order, at most `cap` of them).
+__global__ void adj_hub_kernel(const uint32_t* __restrict__ out, uint64_t N, uint32_t least, uint32_t* __restrict__ hub,
+                               uint32_t* __restrict__ hubs, uint32_t cap, unsigned int* n_hubs) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t step = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < N / 32; w += step) {
         const uint32_t bits = __ballot_sync(kFull, out[w * 32 + lane] >= least);
         if (lane == 0) hub[w] = bits;
+        if (bits == 0) continue;   // uniform
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(n_hubs, __popc(bits));
+        at = __shfl_sync(kFull, at, 0) + __popc(bits & ((1u << lane) - 1u));
+        if ((bits >> lane & 1u) && at < cap) hubs[at] = (uint32_t)w * 32 + lane;
     }
 }
 
@@ -811,20 +819,31 @@ __device__ __forceinline__ bool hook_l1(uint32_t* parent, uint32_t a, uint32_t b
     return hook(parent, hi, lo);
 }
 
-// The hubs, hooked to their first neighbours (hubs themselves, as the lists go).
-constexpr uint32_t kHubLinks = 4;
+// The hubs hooked to their first neighbours (hubs themselves, as the lists go),
+// a neighbour a launch, each followed by pointing every hub at its root: after
+// the first round most hubs share a root and the others' hooks find it in two
+// reads.  (All four neighbours in one launch contend for the few roots left:
+// 370-405 us at Kronecker 25 instead of 245.)
+constexpr uint32_t kHubLinks = 3;
 __global__ void wcc_adj_hub_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
-                                   const uint32_t* __restrict__ hub, uint32_t* parent, uint64_t words,
+                                   const uint32_t* __restrict__ hubs, uint32_t n, uint32_t link, uint32_t* parent,
                                    unsigned long long* unresolved) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t step = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint32_t nth = gridDim.x * blockDim.x;
     uint32_t bad = 0;
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += step) {
-        if (!(__ldg(hub + w) >> lane & 1u)) continue;
-        const uint32_t v = (uint32_t)w * 32 + lane, b = __ldg(off + v), e = min(__ldg(off + v + 1), b + kHubLinks);
-        for (uint32_t i = b; i < e; ++i) bad += !hook_l1(parent, v, __ldg(adj + i));
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nth) {
+        const uint32_t v = __ldg(hubs + i), at = __ldg(off + v) + link;
+        if (at < __ldg(off + v + 1)) bad += !hook_l1(parent, v, __ldg(adj + at));
     }
     warp_add_u64(unresolved, bad);
+}
+
+__global__ void wcc_adj_hub_root_kernel(const uint32_t* __restrict__ hubs, uint32_t n, uint32_t* parent) {
+    const uint32_t nth = gridDim.x * blockDim.x;
+    uint32_t known = ~0u, first;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nth) {
+        const uint32_t v = hubs[i], r = find_root_known(parent, v, known, &first);
+        if (r != first) parent[v] = r;
+    }
 }
 
 // Every other vertex hooked to its first neighbour, four a thread in flight:
@@ -835,7 +854,28 @@ __global__ void wcc_adj_first_kernel(const uint32_t* __restrict__ none, const ui
                                      const uint32_t* __restrict__ adj_out, int directed, uint32_t* parent,
                                      uint8_t* __restrict__ touched, uint64_t N, unsigned long long* unresolved) {
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x, tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t bad = 0;
+    const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    // the pairs whose hook takes a search, run 32 at a time, one per lane (a
+    // few lanes of nearly every warp: searched where they were found, their
+    // chains of dependent reads took 280 of the 480 us at Kronecker 25)
+    __shared__ uint2 s_q[8][64];
+    uint2* q = s_q[threadIdx.x >> 5];
+    uint32_t bad = 0, qn = 0;   // qn: uniform in the warp, below 32 between pushes
+    auto push = [&](bool need, uint32_t v, uint32_t n) {
+        const uint32_t bal = __ballot_sync(kFull, need);
+        if (need) q[qn + __popc(bal & lt)] = make_uint2(v, n);
+        qn += __popc(bal);
+        __syncwarp();
+        if (qn >= 32) {
+            const uint2 mine = q[lane], rest = lane + 32 < qn ? q[lane + 32] : make_uint2(0, 0);
+            __syncwarp();
+            if (lane + 32 < qn) q[lane] = rest;
+            qn -= 32;
+            bad += !hook_l1(parent, mine.x, mine.y);
+            __syncwarp();
+        }
+    };
+    // (N is a multiple of 65,536: the warp stays together)
     for (uint64_t v0 = tid; v0 < N; v0 += 4 * nth) {
         uint32_t n[4], pn[4], rn[4];
         bool link[4];
@@ -859,52 +899,59 @@ __global__ void wcc_adj_first_kernel(const uint32_t* __restrict__ none, const ui
         for (int j = 0; j < 4; ++j) rn[j] = link[j] ? parent[pn[j]] : 0u;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (!link[j]) continue;
             const uint32_t v = (uint32_t)(v0 + j * nth);
             // v is mostly still alone: linked under the neighbour's root at once
-            if (rn[j] == pn[j] && pn[j] < v && atomicCAS(parent + v, v, pn[j]) == v) continue;
-            bad += !hook_l1(parent, v, n[j]);
+            const bool at_once = link[j] && rn[j] == pn[j] && pn[j] < v && atomicCAS(parent + v, v, pn[j]) == v;
+            link[j] = link[j] && !at_once;
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) push(link[j], (uint32_t)(v0 + j * nth), n[j]);
     }
+    if (lane < qn) bad += !hook_l1(parent, q[lane].x, q[lane].y);
     warp_add_u64(unresolved, bad);
 }
 
 // The entries of the vertices outside the largest tree (bit clear in `giant`):
 // the records with both ends in it join nothing new.  A vertex that has joined
 // it meanwhile is done too -- a neighbour still outside has the record in its
-// own list.  A warp per 32-vertex word; short rows a lane each, long ones the
-// warp together.
+// own list.  A warp takes 32 words and compacts their vertices; short rows a
+// lane each, long ones the warp together.
 __global__ void wcc_adj_rest_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
-                                    uint32_t* parent, const uint32_t* __restrict__ giant,
-                                    const uint32_t* __restrict__ root, uint64_t words, unsigned long long* unresolved) {
-    const uint32_t lane = threadIdx.x & 31;
+                                    const uint32_t* __restrict__ none, uint32_t* parent,
+                                    const uint32_t* __restrict__ giant, const uint32_t* __restrict__ root,
+                                    uint64_t words, unsigned long long* unresolved) {
+    __shared__ uint16_t s_list[8][1024];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t step = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const uint32_t c = *root;   // ~0: no tree was found
     uint32_t bad = 0;
     auto joined = [&](uint32_t v) { return c != ~0u && find_root_l1(parent, v) == find_root_l1(parent, c); };
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += step) {
-        const uint32_t g = __ldg(giant + w);
-        if (g == ~0u) continue;   // uniform
-        const uint32_t v = (uint32_t)w * 32 + lane;
-        const bool out = !(g >> lane & 1u);
-        const uint32_t b = out ? __ldg(off + v) : 0u, e = out ? __ldg(off + v + 1) : 0u;
-        const bool is_long = e - b > kProbe;
-        if (!is_long)
-            for (uint32_t i = b; i < e; ++i) {
-                bad += !hook_l1(parent, v, __ldg(adj + i));
-                if ((i - b) % 4 == 0 && joined(v)) break;
-            }
-        uint32_t more = __ballot_sync(kFull, is_long);
-        while (more) {
-            const uint32_t l = __ffs(more) - 1;
-            more &= more - 1;
-            const uint32_t lb = __shfl_sync(kFull, b, l), le = __shfl_sync(kFull, e, l), lv = (uint32_t)w * 32 + l;
-            for (uint32_t i = lb; i < le; i += 32) {   // uniform
-                if (i + lane < le) bad += !hook_l1(parent, lv, __ldg(adj + i + lane));
-                if (__any_sync(kFull, lane == 0 && joined(lv))) break;
+    for (uint64_t w0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; w0 < words; w0 += step * 32) {
+        const uint64_t w = w0 + lane;
+        const uint32_t n = list_bits(s_list[warp], w < words ? ~(__ldg(giant + w) | (none ? __ldg(none + w) : 0u)) : 0u,
+                                     lane);
+        for (uint32_t t = 0; t < n; t += 32) {
+            const bool has = t + lane < n;
+            const uint32_t v = (uint32_t)w0 * 32 + (has ? s_list[warp][t + lane] : 0u);
+            const uint32_t b = has ? __ldg(off + v) : 0u, e = has ? __ldg(off + v + 1) : 0u;
+            const bool is_long = e - b > kProbe;
+            if (!is_long)
+                for (uint32_t i = b; i < e; ++i) {
+                    bad += !hook_l1(parent, v, __ldg(adj + i));
+                    if ((i - b) % 4 == 0 && joined(v)) break;
+                }
+            uint32_t more = __ballot_sync(kFull, is_long);
+            while (more) {
+                const uint32_t l = __ffs(more) - 1;
+                more &= more - 1;
+                const uint32_t lb = __shfl_sync(kFull, b, l), le = __shfl_sync(kFull, e, l), lv = __shfl_sync(kFull, v, l);
+                for (uint32_t i = lb; i < le; i += 32) {   // uniform
+                    if (i + lane < le) bad += !hook_l1(parent, lv, __ldg(adj + i + lane));
+                    if (__any_sync(kFull, lane == 0 && joined(lv))) break;
+                }
             }
         }
-        __syncwarp();
+        __syncwarp();   // s_list is rewritten
     }
     warp_add_u64(unresolved, bad);
 }
@@ -961,7 +1008,9 @@ gs_status adj_build(gs_graph* g) {
     if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.off_in, (N + 1) * 4);
     if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.adj_in, std::max<uint64_t>(1, dir ? E : 2 * E) * 4);
     if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.none, words * 4);
+    const uint32_t hub_cap = (uint32_t)(N / 2);
     if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.hub, words * 4);
+    if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.hubs, (uint64_t)hub_cap * 4);
     if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.first_in, N * 4);
     if (st == GS_OK && dir) st = gs_graph_alloc(g, (void**)&A.off_out, (N + 1) * 4);
     if (st == GS_OK && dir) st = gs_graph_alloc(g, (void**)&A.adj_out, std::max<uint64_t>(1, E) * 4);
@@ -1009,7 +1058,11 @@ gs_status adj_build(gs_graph* g) {
             // four times the mean: at Kronecker 26 the 2 % of the vertices that
             // hold about three quarters of the entries
             const uint32_t least = (uint32_t)std::max<uint64_t>(2, 4 * A.n_in / std::max<uint64_t>(1, A.n_cand));
-            adj_hub_kernel<<<blocks_for(N, ctx), 256, 0, q>>>(A.off_out, N, least, A.hub);
+            // a hub has four times the mean of the vertices with entries, so at
+            // most a quarter of those are hubs
+            adj_hub_kernel<<<blocks_for(N, ctx), 256, 0, q>>>(A.off_out, N, least, A.hub, A.hubs, hub_cap,
+                                                              (unsigned int*)tmp + 2);
+            run(cudaMemcpyAsync(ctx->h_scalars, tmp, 16, cudaMemcpyDeviceToHost, q));
         }
         run(cub::DeviceScan::ExclusiveSum(cub_tmp, scan_bytes, (const uint32_t*)A.off_in, A.off_in, N + 1, q));
         if (dir) run(cub::DeviceScan::ExclusiveSum(cub_tmp, scan_bytes, (const uint32_t*)A.off_out, A.off_out, N + 1, q));
@@ -1022,6 +1075,7 @@ gs_status adj_build(gs_graph* g) {
         }
         run(cudaGetLastError());
         run(cudaStreamSynchronize(q));
+        A.n_hub = std::min<uint64_t>(((const uint32_t*)ctx->h_scalars)[2], hub_cap);
         ctx->launches += 14;
         if (e != cudaSuccess) st = gs_cuda_fail(ctx, e, "adjacency lists");
     }
@@ -1045,6 +1099,7 @@ void gs_adj_free(gs_graph* g) {
     gs_graph_release(g, A.first_in);
     gs_graph_release(g, A.none);
     gs_graph_release(g, A.hub);
+    gs_graph_release(g, A.hubs);
     const uint32_t credit = A.credit;
     A = gs_adj();
     A.credit = credit;
@@ -1061,7 +1116,7 @@ bool gs_adj_ready(gs_graph* g, uint32_t sweeps) {
     }
     A.refused = true;   // unless all goes well
     if (n_lists(g) >= (1ull << 32) - (1ull << 20)) return false;   // 32-bit offsets
-    const uint64_t keep = n_lists(g) * 4 + g->N * (g->directed ? 13 : 9);
+    const uint64_t keep = n_lists(g) * 4 + g->N * (g->directed ? 15 : 11);
     if (ctx->budget && 4 * g->E + keep > ctx->budget) return false;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
@@ -1164,20 +1219,26 @@ gs_status wcc_adj_hook(gs_state* s, void (*vote)(gs_state*), unsigned long long*
     gs_ctx* ctx = g->ctx;
     const gs_adj& A = g->adj;
     const uint64_t N = g->N, words = N / 32;
-    const uint32_t grid = gs_grid_size(ctx, 8), by_word = (uint32_t)std::min<uint64_t>((words + 7) / 8, grid);
-    wcc_adj_hub_kernel<<<by_word, 256, 0, ctx->stream>>>(A.off_in, A.adj_in, A.hub, s->d_parent, words, unresolved);
+    const uint32_t grid = gs_grid_size(ctx, 8), by_block = (uint32_t)std::min<uint64_t>((words + 255) / 256, grid);
+    const uint32_t by_hub = (uint32_t)std::min<uint64_t>((A.n_hub + 255) / 256, grid);
+    for (uint32_t link = 0; link < kHubLinks && A.n_hub; ++link) {
+        wcc_adj_hub_kernel<<<by_hub, 256, 0, ctx->stream>>>(A.off_in, A.adj_in, A.hubs, (uint32_t)A.n_hub, link,
+                                                            s->d_parent, unresolved);
+        wcc_adj_hub_root_kernel<<<by_hub, 256, 0, ctx->stream>>>(A.hubs, (uint32_t)A.n_hub, s->d_parent);
+        ctx->launches += 2;
+    }
     wcc_adj_first_kernel<<<(uint32_t)std::min<uint64_t>((N + 1023) / 1024, grid), 256, 0, ctx->stream>>>(
         A.none, A.first_in, A.hub, A.off_out, A.adj_out, g->directed, s->d_parent, s->d_touched, N, unresolved);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     vote(s);
     const uint32_t* root = s->d_giant + words;
-    wcc_adj_rest_kernel<<<by_word, 256, 0, ctx->stream>>>(A.off_in, A.adj_in, s->d_parent, s->d_giant, root, words,
-                                                          unresolved);
+    wcc_adj_rest_kernel<<<by_block, 256, 0, ctx->stream>>>(A.off_in, A.adj_in, A.none, s->d_parent, s->d_giant, root,
+                                                           words, unresolved);
     if (g->directed)
-        wcc_adj_rest_kernel<<<by_word, 256, 0, ctx->stream>>>(A.off_out, A.adj_out, s->d_parent, s->d_giant, root, words,
-                                                              unresolved);
+        wcc_adj_rest_kernel<<<by_block, 256, 0, ctx->stream>>>(A.off_out, A.adj_out, nullptr, s->d_parent, s->d_giant,
+                                                               root, words, unresolved);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
-    ctx->launches += g->directed ? 4 : 3;
+    ctx->launches += g->directed ? 3 : 2;
     return GS_OK;
 }
 

@@ -162,6 +162,8 @@ struct gs_adj {
     uint32_t* first_in = nullptr;    // N: every vertex's first in-entry
     uint32_t* none = nullptr;        // N / 32 words: vertices without in-entries
     uint32_t* hub = nullptr;         // N / 32 words: vertices with over four times the mean entries
+    uint32_t* hubs = nullptr;        // and their list
+    uint64_t n_hub = 0;
     uint64_t n_in = 0, n_cand = 0;   // in-entries, vertices that have some
     uint32_t credit = 0;             // sweeps of the grid done by whole queries
     bool built = false, refused = false;
@@ -284,6 +286,7 @@ struct gs_state {
     uint32_t* d_parent = nullptr;    // N
     uint8_t* d_touched = nullptr;    // N
     uint32_t* d_giant = nullptr;     // N/32 + 2 words: largest sampled tree's bitmap, then its root
+    bool wcc_touched = false;        // d_touched is complete (hooked on adjacency lists)
     bool wcc_giant = false;          // d_giant was built by this run's first sweep
     // k-core
     int32_t* d_deg = nullptr;        // N

@@ -164,11 +164,8 @@ __device__ __forceinline__ uint32_t find_root(const uint32_t* parent, uint32_t v
 // roots: `known` is a root this thread found before, and a vertex pointing at
 // it needs no second load.  After pointer jumping nearly every vertex of the
 // largest tree points at one root, whose own entry every warp of the grid
-// would otherwise read from a single L2 slice.  *first = parent[v].
-__device__ __forceinline__ uint32_t find_root_known(const uint32_t* parent, uint32_t v, uint32_t& known,
-                                                    uint32_t* first) {
-    uint32_t p = __ldcg(parent + v);
-    *first = p;
+// would otherwise read from a single L2 slice.  p = parent[v].
+__device__ __forceinline__ uint32_t find_root_from(const uint32_t* parent, uint32_t v, uint32_t p, uint32_t& known) {
     if (p == v || p == known) return p;
     while (true) {
         const uint32_t pp = __ldcg(parent + p);
@@ -177,6 +174,13 @@ __device__ __forceinline__ uint32_t find_root_known(const uint32_t* parent, uint
     }
     known = p;
     return p;
+}
+
+// The same from v alone.  *first = parent[v].
+__device__ __forceinline__ uint32_t find_root_known(const uint32_t* parent, uint32_t v, uint32_t& known,
+                                                    uint32_t* first) {
+    *first = __ldcg(parent + v);
+    return find_root_from(parent, v, *first, known);
 }
 
 // find_root with path halving: every vertex passed on the way points to its

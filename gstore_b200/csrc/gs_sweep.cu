@@ -327,14 +327,22 @@ __global__ void iota_kernel(uint32_t* parent, uint64_t N) {
     for (uint64_t v = tid; v < N; v += nth) parent[v] = (uint32_t)v;
 }
 
-// Pointer jumping (wcc.cpp:372-390): every vertex points at its root.
+// Pointer jumping (wcc.cpp:372-390): every vertex points at its root.  Four
+// neighbouring vertices a thread (N is a multiple of 65,536), here and in the
+// two kernels below: one vertex a thread leaves one dependent chain in flight
+// (72 -> 42 us at Kronecker 25; 91 -> 69 and 136 -> 59 for the two).
 __global__ void compress_kernel(uint32_t* parent, uint64_t N) {
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
-    uint32_t known = ~0u, first;
-    for (uint64_t v = tid; v < N; v += nth) {
-        const uint32_t r = find_root_known(parent, (uint32_t)v, known, &first);
-        if (r != first) parent[v] = r;
+    uint32_t known = ~0u;
+    for (uint64_t i = tid; i < N / 4; i += nth) {
+        const uint4 p = __ldcg(reinterpret_cast<const uint4*>(parent) + i);
+        const uint32_t q[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t v = (uint32_t)(i * 4 + j), r = find_root_from(parent, v, q[j], known);
+            if (r != q[j]) parent[v] = r;
+        }
     }
 }
 
@@ -368,20 +376,28 @@ __global__ void __launch_bounds__(kGiantSamples) wcc_giant_root_kernel(const uin
 }
 
 // Pointer jumping as compress_kernel, and the bitmap of the vertices whose
-// root is *root (the largest sampled tree): bit v & 31 of word v >> 5.
-// Warps take whole 32-vertex words (N is a multiple of 65,536).
+// root is *root (the largest sampled tree): bit v & 31 of word v >> 5, eight
+// lanes to a word.
 __global__ void wcc_compress_giant_kernel(uint32_t* parent, uint32_t* giant, const uint32_t* root, uint64_t N) {
     const uint32_t c = *root;
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nwords = N >> 5;
-    const uint64_t step = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint32_t known = c, first;   // c is a root: the sampled pass is over
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nwords; w += step) {
-        const uint32_t v = (uint32_t)(w * 32 + lane);
-        const uint32_t r = find_root_known(parent, v, known, &first);
-        if (r != first) parent[v] = r;
-        const uint32_t bits = __ballot_sync(kFull, r == c);
-        if (lane == 0) giant[w] = bits;
+    const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t known = c;   // c is a root: the sampled pass is over
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N / 4; i += nth) {   // whole warps
+        const uint4 p = __ldcg(reinterpret_cast<const uint4*>(parent) + i);
+        const uint32_t q[4] = {p.x, p.y, p.z, p.w};
+        uint32_t bits = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t v = (uint32_t)(i * 4 + j), r = find_root_from(parent, v, q[j], known);
+            if (r != q[j]) parent[v] = r;
+            bits |= (r == c ? 1u : 0u) << j;
+        }
+        bits <<= 4 * (lane & 7);
+        bits |= __shfl_xor_sync(kFull, bits, 1);
+        bits |= __shfl_xor_sync(kFull, bits, 2);
+        bits |= __shfl_xor_sync(kFull, bits, 4);
+        if ((lane & 7) == 0) giant[i / 8] = bits;
     }
 }
 
@@ -390,15 +406,20 @@ __global__ void wcc_label_kernel(const uint32_t* parent, const uint8_t* touched,
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
     uint64_t local = 0;
-    uint32_t known = ~0u, first;
-    for (uint64_t v = tid; v < N; v += nth) {
-        if (!touched[v]) {
-            out[v] = 0xFFFFFFFFu;  // invalid_cid, wcc.cpp:54
-            continue;
+    uint32_t known = ~0u;
+    for (uint64_t i = tid; i < N / 4; i += nth) {
+        const uint4 p = __ldcg(reinterpret_cast<const uint4*>(parent) + i);
+        const uchar4 t = reinterpret_cast<const uchar4*>(touched)[i];
+        const uint32_t q[4] = {p.x, p.y, p.z, p.w};
+        const bool named[4] = {t.x != 0, t.y != 0, t.z != 0, t.w != 0};
+        uint32_t l[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t v = (uint32_t)(i * 4 + j);
+            l[j] = named[j] ? find_root_from(parent, v, q[j], known) : 0xFFFFFFFFu;  // invalid_cid, wcc.cpp:54
+            local += l[j] == v && named[j];
         }
-        const uint32_t r = find_root_known(parent, (uint32_t)v, known, &first);
-        out[v] = r;
-        local += (r == v);
+        reinterpret_cast<uint4*>(out)[i] = make_uint4(l[0], l[1], l[2], l[3]);
     }
     warp_add_u64(count, local);
 }
@@ -668,6 +689,7 @@ gs_status wcc_init(gs_state* s) {
     gs_ctx* ctx = g->ctx;
     if (!s->d_parent) GS_TRY(gs_state_alloc(s, (void**)&s->d_parent, g->N * 4));
     if (!s->d_touched) GS_TRY(gs_state_alloc(s, (void**)&s->d_touched, g->N));
+    s->wcc_touched = false;
     iota_kernel<<<blocks_for(g->N, ctx), kThreads, 0, ctx->stream>>>(s->d_parent, g->N);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
@@ -711,6 +733,7 @@ gs_status wcc_sweep_launch(gs_state* s) {
         if (!s->d_giant) GS_TRY(gs_state_alloc(s, (void**)&s->d_giant, (g->N / 32 + 2) * 4));
         if (g->adj.built) {   // not dropped by that allocation
             s->wcc_giant = false;
+            s->wcc_touched = true;   // by its entries, every vertex of a record
             gs_timer_begin(ctx);
             GS_TRY(wcc_adj_hook(s, wcc_vote, (unsigned long long*)ctx->d_scalars));
             gs_timer_end(ctx, GS_ALGO_WCC, bytes);
@@ -776,11 +799,14 @@ gs_status gs_wcc_labels(gs_state* s, uint32_t* d_out, uint64_t* count) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
     GS_TRY(zero_scalar(ctx));
-    wcc_mark_touched<<<blocks_for(g->N, ctx), kThreads, 0, ctx->stream>>>(s->d_parent, s->d_touched, g->N);
+    if (!s->wcc_touched) {
+        wcc_mark_touched<<<blocks_for(g->N, ctx), kThreads, 0, ctx->stream>>>(s->d_parent, s->d_touched, g->N);
+        ctx->launches++;
+    }
     wcc_label_kernel<<<blocks_for(g->N, ctx), kThreads, 0, ctx->stream>>>(
         s->d_parent, s->d_touched, d_out, g->N, (unsigned long long*)ctx->d_scalars);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
-    ctx->launches += 2;
+    ctx->launches++;
     return read_scalar(ctx, count);
 }
 

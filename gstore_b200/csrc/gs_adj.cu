@@ -184,22 +184,6 @@ __device__ __forceinline__ AdjItem load_item(const AdjItem* p) {
     return AdjItem{__ldcg(&p->v), __ldcg(&p->beg), __ldcg(&p->end)};
 }
 
-// The set bits of the warp's 32 words, in order, into list; how many.
-__device__ __forceinline__ uint32_t list_bits(uint16_t* list, uint32_t x, uint32_t lane) {
-    uint32_t at = __popc(x);
-    const uint32_t own = at;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, at, o);
-        if (lane >= (uint32_t)o) at += y;
-    }
-    const uint32_t sum = __shfl_sync(kFull, at, 31);
-    at -= own;
-    for (; x; x &= x - 1) list[at++] = (uint16_t)(lane * 32 + __ffs(x) - 1);
-    __syncwarp();
-    return sum;
-}
-
 struct BfsCtl {
     unsigned long long total[256];   // vertices found per level ([0]: the root)
     unsigned long long edges[256];   // their out-entries (after a bottom-up level: an estimate)

@@ -66,6 +66,22 @@ __device__ __forceinline__ void warp_add_u64(unsigned long long* dst, uint64_t v
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(dst, (unsigned long long)v);
 }
 
+// The set bits of the warp's 32 words, in order, into list; how many.
+__device__ __forceinline__ uint32_t list_bits(uint16_t* list, uint32_t x, uint32_t lane) {
+    uint32_t at = __popc(x);
+    const uint32_t own = at;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, at, o);
+        if (lane >= (uint32_t)o) at += y;
+    }
+    const uint32_t sum = __shfl_sync(kFull, at, 31);
+    at -= own;
+    for (; x; x &= x - 1) list[at++] = (uint16_t)(lane * 32 + __ffs(x) - 1);
+    __syncwarp();
+    return sum;
+}
+
 // ------------------------------------------------------------ grid barrier --
 constexpr uint64_t kBarrierNs = 4000000000ull;   // 4 s
 

@@ -269,6 +269,7 @@ struct gs_state {
     uint32_t* d_visited = nullptr;   // N/32 words: discovered-this-sweep bitmap
     uint64_t* d_error = nullptr;     // bounded-wait failure flag
     uint32_t* d_ticket = nullptr;    // BFS sweep: run ticket, finished CTAs
+    unsigned long long* d_count = nullptr;   // BFS finalize: vertices found, finished CTAs (zero between levels)
     uint8_t* d_dead = nullptr;       // BFS: per unit, chunks with no record left to discover anything
     bool marking = false;            // BFS: dead chunks are being marked (and skipped)
     bool sweep_mark = false, sweep_skip = false;   // BFS: this level's mode (set per sweep)

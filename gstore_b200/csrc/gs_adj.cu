@@ -988,16 +988,16 @@ gs_status adj_build(gs_graph* g) {
     const uint64_t u4 = ((uint64_t)U + 63) & ~63ull;
     const size_t tmp_bytes = 256 + cub_bytes + u4 * 4 * 5 + N * 4 * (dir ? 3 : 2);
     char* tmp = nullptr;
-    gs_status st = gs_pool_get(ctx, tmp_bytes, (void**)&tmp);
-    if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.off_in, (N + 1) * 4);
-    if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.adj_in, std::max<uint64_t>(1, dir ? E : 2 * E) * 4);
-    if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.none, words * 4);
+    gs_status st = gs_dev_alloc(ctx, (void**)&tmp, tmp_bytes);
+    if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.off_in, (N + 1) * 4);
+    if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.adj_in, std::max<uint64_t>(1, dir ? E : 2 * E) * 4);
+    if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.none, words * 4);
     const uint32_t hub_cap = (uint32_t)(N / 2);
-    if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.hub, words * 4);
-    if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.hubs, (uint64_t)hub_cap * 4);
-    if (st == GS_OK) st = gs_graph_alloc(g, (void**)&A.first_in, N * 4);
-    if (st == GS_OK && dir) st = gs_graph_alloc(g, (void**)&A.off_out, (N + 1) * 4);
-    if (st == GS_OK && dir) st = gs_graph_alloc(g, (void**)&A.adj_out, std::max<uint64_t>(1, E) * 4);
+    if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.hub, words * 4);
+    if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.hubs, (uint64_t)hub_cap * 4);
+    if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.first_in, N * 4);
+    if (st == GS_OK && dir) st = gs_dev_alloc(ctx, (void**)&A.off_out, (N + 1) * 4);
+    if (st == GS_OK && dir) st = gs_dev_alloc(ctx, (void**)&A.adj_out, std::max<uint64_t>(1, E) * 4);
     cudaError_t e = cudaSuccess;
     if (st == GS_OK) {
         if (!dir) {
@@ -1063,7 +1063,7 @@ gs_status adj_build(gs_graph* g) {
         ctx->launches += 14;
         if (e != cudaSuccess) st = gs_cuda_fail(ctx, e, "adjacency lists");
     }
-    gs_pool_put(ctx, tmp, tmp_bytes);
+    gs_dev_free(tmp);   // (waits for the build)
     if (st != GS_OK) {
         gs_adj_free(g);
         return st;
@@ -1076,14 +1076,12 @@ gs_status adj_build(gs_graph* g) {
 
 void gs_adj_free(gs_graph* g) {
     gs_adj& A = g->adj;
-    if (A.off_out != A.off_in) gs_graph_release(g, A.off_out);
-    if (A.adj_out != A.adj_in) gs_graph_release(g, A.adj_out);
-    gs_graph_release(g, A.off_in);
-    gs_graph_release(g, A.adj_in);
-    gs_graph_release(g, A.first_in);
-    gs_graph_release(g, A.none);
-    gs_graph_release(g, A.hub);
-    gs_graph_release(g, A.hubs);
+    // not pool blocks: their gigabytes would keep the records of the next
+    // uploads out of the pool
+    if (A.off_out != A.off_in) gs_dev_free(A.off_out);
+    if (A.adj_out != A.adj_in) gs_dev_free(A.adj_out);
+    for (void* p : {(void*)A.off_in, (void*)A.adj_in, (void*)A.first_in, (void*)A.none, (void*)A.hub, (void*)A.hubs})
+        gs_dev_free(p);
     const uint32_t credit = A.credit;
     A = gs_adj();
     A.credit = credit;

@@ -20,7 +20,7 @@
 // independent ones per lane in flight and works on compacted lists of the
 // vertices concerned instead of on words with a few bits set.
 //
-// The lists cost 8 bytes per record and 11 per vertex of HBM, and building
+// The lists cost 8 bytes per record and 9 per vertex of HBM, and building
 // them takes about 7 such queries' time (45 ms at Kronecker 26, 22 at 25).  So a
 // graph gets them once its queries have swept it kAdjBuild times, eight BFS or
 // k-core queries or eleven WCC (gs_adj_ready: a graph that is queried only a
@@ -995,7 +995,7 @@ gs_status adj_build(gs_graph* g) {
     if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.off_in, (N + 1) * 4);
     if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.adj_in, std::max<uint64_t>(1, dir ? E : 2 * E) * 4);
     if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.none, words * 4);
-    const uint32_t hub_cap = (uint32_t)(N / 2);
+    const uint32_t hub_cap = (uint32_t)(N / 32);
     if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.hub, words * 4);
     if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.hubs, (uint64_t)hub_cap * 4);
     if (st == GS_OK) st = gs_dev_alloc(ctx, (void**)&A.first_in, N * 4);
@@ -1042,11 +1042,12 @@ gs_status adj_build(gs_graph* g) {
         run(cudaMemcpyAsync(ctx->h_scalars, d_some, 8, cudaMemcpyDeviceToHost, q));
         if (run(cudaStreamSynchronize(q))) {
             A.n_cand = ctx->h_scalars[0];
-            // four times the mean: at Kronecker 26 the 2 % of the vertices that
-            // hold about three quarters of the entries
-            const uint32_t least = (uint32_t)std::max<uint64_t>(2, 4 * A.n_in / std::max<uint64_t>(1, A.n_cand));
-            // a hub has four times the mean of the vertices with entries, so at
-            // most a quarter of those are hubs
+            // 32 times the mean: the bottom-up level that counts has a frontier of
+            // the largest hubs only (17 roots at Kronecker 26, mean: 4 times the
+            // mean 0.95 ms, 8 0.93, 16 0.90, 32 and 64 0.84)
+            const uint32_t least = (uint32_t)std::min<uint64_t>(
+                32 * ((A.n_in + A.n_cand - 1) / std::max<uint64_t>(1, A.n_cand)), 0xFFFFFFFFu);
+            // (so at most one vertex in 32 is a hub)
             adj_hub_kernel<<<blocks_for(N, ctx), 256, 0, q>>>(A.off_out, N, least, A.hub, A.hubs, hub_cap,
                                                               (unsigned int*)tmp + 2);
             run(cudaMemcpyAsync(ctx->h_scalars, tmp, 16, cudaMemcpyDeviceToHost, q));
@@ -1101,7 +1102,7 @@ bool gs_adj_ready(gs_graph* g, uint32_t sweeps) {
     }
     A.refused = true;   // unless all goes well
     if (n_lists(g) >= (1ull << 32) - (1ull << 20)) return false;   // 32-bit offsets
-    const uint64_t keep = n_lists(g) * 4 + g->N * (g->directed ? 15 : 11);
+    const uint64_t keep = n_lists(g) * 4 + g->N * (g->directed ? 13 : 9);
     if (ctx->budget && 4 * g->E + keep > ctx->budget) return false;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;

@@ -161,7 +161,7 @@ struct gs_adj {
     uint32_t *off_out = nullptr, *adj_out = nullptr;
     uint32_t* first_in = nullptr;    // N: every vertex's first in-entry
     uint32_t* none = nullptr;        // N / 32 words: vertices without in-entries
-    uint32_t* hub = nullptr;         // N / 32 words: vertices with over four times the mean entries
+    uint32_t* hub = nullptr;         // N / 32 words: vertices with 32 times the mean entries and more
     uint32_t* hubs = nullptr;        // and their list
     uint64_t n_hub = 0;
     uint64_t n_in = 0, n_cand = 0;   // in-entries, vertices that have some

@@ -202,7 +202,7 @@ gs_status gs_finalize(gs_state* s, int64_t* frontier_out, int* done_out);
 /* Sweep + finalize until done, all on the device (one 8-byte read per step).
  * steps_out: number of sweeps.  Once whole queries have swept a resident graph
  * often enough (about eight BFS or k-core queries), and while HBM has room, the
- * graph also keeps its records as adjacency lists (8 bytes per record and 12
+ * graph also keeps its records as adjacency lists (8 bytes per record and 9
  * per vertex until gs_graph_free, dropped earlier when an allocation fails), and BFS,
  * WCC and k-core run on those: the same results and step counts, in one to
  * eight launches. */

@@ -105,10 +105,11 @@ struct gs_pr_layout {
 // PageRank propagation-blocked layout (gs_pr_blocked.cu): one entry per
 // (record, direction), sorted by (source slice, destination bin); u16 offsets
 // of the source in its slice and of the destination in its bin, one float
-// value per entry written by the gather pass, and for the accumulate pass the
-// list of every bin's 8-entry groups (its blocks in slice order).
+// value per entry written by the gather pass, and for the second pass the list
+// of every bin's 8-entry groups (its blocks in slice order).
 constexpr int kPbSrcBits = 14;   // source slice: 16,384 vertices (x staged in shared memory)
 constexpr int kPbDstBits = 14;   // destination bin: 16,384 vertices (sums in shared memory)
+constexpr uint64_t kPbPullSources = 256ull << kPbSrcBits;   // most vertices of a graph with pulled bins
 struct gs_pb_item1 {             // gather item: entries [e0, e0 + n) of source slice `slice`
     uint64_t e0;
     uint32_t n, slice;
@@ -128,6 +129,13 @@ struct gs_pb_layout {
     gs_pb_item1* d_items1 = nullptr;
     gs_pb_item2* d_items2 = nullptr;
     uint64_t n_entries = 0, n_groups = 0, n_items1 = 0, n_items2 = 0;
+    // pulled bins (instead of d_dst and d_items2): n_items2 bins of bin_rows
+    // destinations, which a lane each sums
+    uint32_t bin_rows = 0;               // a multiple of 32; 0: accumulated bins
+    uint32_t* d_bin_group = nullptr;     // first group of every bin, and the end
+    uint32_t* d_strip = nullptr;         // first step of every 32 rows of one bin, and the end
+    uint16_t* d_perm = nullptr;          // destination offset in its bin of every row
+    uint16_t* d_idx = nullptr;           // per step and lane the bin's positions of 4 entries
     bool built = false;
 };
 

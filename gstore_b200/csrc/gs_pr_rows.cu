@@ -36,10 +36,11 @@
 // moved per entry, a shared-memory atomic per run of destinations): Kronecker
 // 20 / 24 / 26, edge factor 16: 81 / 1,045 / 5,900 us against 146 / 1,862 /
 // 8,010; the layout keeps 4.4 bytes per entry instead of 12.5.  Without hubs
-// (uniform random, 3 M vertices, 24 M entries) 153 against 130: rl_worth.
+// (uniform random, 3 M vertices, 24 M entries) 153 against 100: rl_worth.
 // At Kronecker 23 the pull reads 28 % of its entries' sources through L2 and
 // its L1 runs at 70 % of its peak; of DRAM it needs about a third.
 #include "gs_internal.cuh"
+#include "gs_temps.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -458,77 +459,16 @@ __global__ void rl_fill_kernel(const RlGroups G, uint32_t n_slices, const uint32
 // falls into panels they have enough entries in.  0.9 and 5.0 fit the sweeps
 // above (Kronecker 24: 2.0 estimated, 1.8 measured; 26: 3.0 and 2.7; uniform,
 // 3 M vertices: 5.0 and 5.4); propagation blocking measured 3.5-4.9, the row
-// slices 7.5 and more.
+// slices 7.5 and more.  Up to kPbPullSources vertices its bins may be pulled:
+// 18.4 us per iteration against the row lists' 19.6 at 50,000 vertices and 16
+// entries each, uniform (3.1 estimated), 20.5 against 20.6 at 80,000, 20.6
+// against 24.5 at 120,000 (3.5), 32.4 against 41.4 at 400,000.
 bool rl_worth(const gs_graph* g, uint64_t n_ent, const unsigned long long at[4]) {
     const double n = (double)n_ent, hot = at[0] / n, all = at[1] / n, l2 = at[2] / n, heavy = at[3] / n;
     const double staged = hot + 0.8 * heavy * (all - hot), far = 1.0 - l2;
     const double pull = 0.9 * staged + 5.0 * std::max(0.0, l2 - staged) + 24.0 * far;
-    return pull <= (pb_layout_wanted(g) ? 3.7 : 7.5);
-}
-
-inline uint32_t grid_for(uint64_t n, const gs_ctx* ctx) {
-    const uint64_t b = (n + 255) / 256;
-    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(b, gs_grid_size(ctx, 16)));
-}
-
-int bits_for(uint64_t n) {   // bits that hold 0 .. n - 1, at least 1
-    int b = 1;
-    while ((1ull << b) < n) ++b;
-    return b;
-}
-
-// Device buffers of a build: carved from one block (a cudaMalloc and a
-// cudaFree per buffer took 10 of 18 ms at 24 M entries), freed together when
-// the build ends; a buffer that no longer fits gets a block of its own.
-struct Temps {
-    gs_ctx* ctx;
-    std::vector<void*> all;
-    char* top = nullptr;
-    char* end = nullptr;
-    explicit Temps(gs_ctx* c) : ctx(c) {}
-    ~Temps() {
-        cudaStreamSynchronize(ctx->stream);
-        for (void* p : all) gs_dev_free(p);
-    }
-    gs_status reserve(uint64_t bytes) {
-        GS_TRY(gs_dev_alloc(ctx, (void**)&top, bytes));
-        all.push_back(top);
-        end = top + bytes;
-        return GS_OK;
-    }
-    // Buffers to come are carved from [p, p + bytes), which holds nothing needed.
-    void reuse(void* p, uint64_t bytes) {
-        if (bytes <= (uint64_t)(end - top)) return;
-        top = (char*)p;
-        end = top + (bytes & ~255ull);
-    }
-    template <class T>
-    gs_status get(T** out, uint64_t n) {
-        const uint64_t bytes = (std::max<uint64_t>(1, n) * sizeof(T) + 255) & ~255ull;
-        if (bytes <= (uint64_t)(end - top)) {
-            *out = (T*)top;
-            top += bytes;
-            return GS_OK;
-        }
-        GS_TRY(gs_dev_alloc(ctx, (void**)out, bytes));
-        all.push_back(*out);
-        return GS_OK;
-    }
-};
-
-// cub call in two steps: size, then work, with scratch from T that the next
-// buffer (in stream order) may overwrite.
-template <class F>
-gs_status cub_run(Temps& T, const char* what, F call) {
-    size_t bytes = 0;
-    GS_CHECK_CUDA(T.ctx, call(nullptr, bytes));
-    char *mark = T.top, *mark_end = T.end, *tmp = nullptr;
-    GS_TRY(T.get(&tmp, bytes));
-    cudaError_t e = call(tmp, bytes);
-    T.ctx->launches++;
-    if (e != cudaSuccess) return gs_cuda_fail(T.ctx, e, what);
-    if (T.end == mark_end) T.top = mark;
-    return GS_OK;
+    if (!pb_layout_wanted(g)) return pull <= 7.5;
+    return pull <= (g->N <= kPbPullSources ? 3.4 : 3.7);
 }
 
 // Vertices by falling count: order[i], and counts in that order.
@@ -548,13 +488,6 @@ gs_status sort_by_count(Temps& T, const uint32_t* count, uint64_t N, uint32_t** 
     rl_rank_kernel<<<grid_for(N, ctx), 256, 0, ctx->stream>>>(*order, N, *rank);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     ctx->launches += 2;
-    return GS_OK;
-}
-
-template <class T>
-gs_status to_host(gs_ctx* ctx, T* dst, const T* src, uint64_t n) {
-    GS_CHECK_CUDA(ctx, cudaMemcpyAsync(dst, src, n * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return GS_OK;
 }
 

@@ -83,8 +83,8 @@ __global__ void scatter_kernel(const uint2* __restrict__ pairs, uint64_t n, uint
 //   * Counters in global memory, one per tile, take tens of thousands of
 //     atomics on the same few addresses, and slots taken one by one scatter
 //     single records.  Here a CTA takes a stretch of the edges, counts it in
-//     shared memory and reserves each bucket's slots once, so that its records
-//     of a bucket lie side by side.
+//     shared memory and gets each bucket's slots in one piece, so that its
+//     records of a bucket lie side by side.
 //   * A segmented sort gives a segment to a CTA, which needs four passes over
 //     memory for one that does not fit its shared memory: 1.7 ms for the three
 //     tiles of 0.8 M edges over 100,003 vertices.  Slices are small (about
@@ -92,7 +92,7 @@ __global__ void scatter_kernel(const uint2* __restrict__ pairs, uint64_t n, uint
 //   * But not for their own sake: the 2,080 tiles of Kronecker 22 cut into
 //     33,280 slices took 1.82 ms to scatter (shorter stretches) and 2.50 to
 //     sort instead of 0.98 and 2.13.
-// 67 M edges of Kronecker 22, ms: count 1.60 -> 0.94, scatter 1.89 -> 0.98, sort
+// 67 M edges of Kronecker 22, ms: count 1.60 -> 0.94, scatter 1.89 -> 0.81, sort
 // 2.14 as before; 0.8 M edges over 100,003 vertices, all of it: 2.67 -> 0.48.  What
 // is left of the count are the two random degree atomics per edge (~180 G/s).
 constexpr uint32_t kMaxBuckets = 49152;        // 192 KB of counters
@@ -114,17 +114,21 @@ __device__ __forceinline__ uint32_t bucket_of(uint32_t a, uint32_t b, const Buck
     return (bucket_tile(a >> kTileBits, b >> kTileBits, B) << B.bits) | ((b & 0xFFFFu) >> (kTileBits - B.bits));
 }
 
+// A CTA counts the stretch of `per` edges that it will scatter.  Table: its
+// counts go to counts[t * gridDim + CTA], else they are added to counts[t].
+template <bool Table>
 __global__ void __launch_bounds__(kBucketThreads, 1)
-    bucket_count_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t V, const Buckets B,
+    bucket_count_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t per, uint64_t V, const Buckets B,
                         uint32_t* __restrict__ counts, int32_t* __restrict__ deg, int* bad) {
     extern __shared__ uint32_t s_count[];
     for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads) s_count[t] = 0;
     __syncthreads();
-    const uint64_t nth = (uint64_t)gridDim.x * kBucketThreads;
-    for (uint64_t k = (uint64_t)blockIdx.x * kBucketThreads + threadIdx.x; k < n; k += 4 * nth) {
+    const uint64_t lo = blockIdx.x * per, hi = lo + per < n ? lo + per : n;
+    for (uint64_t k = lo + threadIdx.x; k < hi; k += 4 * kBucketThreads) {
         uint2 e[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) e[j] = k + j * nth < n ? __ldcs(pairs + k + j * nth) : make_uint2(0, 0);
+        for (int j = 0; j < 4; ++j)
+            e[j] = k + j * kBucketThreads < hi ? __ldcs(pairs + k + j * kBucketThreads) : make_uint2(0, 0);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (e[j].x == e[j].y) continue;  // is_self_loop
@@ -139,11 +143,23 @@ __global__ void __launch_bounds__(kBucketThreads, 1)
         }
     }
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads)
-        if (s_count[t]) atomicAdd(counts + t, s_count[t]);
+    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads) {
+        if (Table) counts[(uint64_t)t * gridDim.x + blockIdx.x] = s_count[t];
+        else if (s_count[t]) atomicAdd(counts + t, s_count[t]);
+    }
 }
 
-// cursor: the buckets' starts; on return their ends.
+// starts[t] = the scanned table's entry of bucket t's first stretch.
+__global__ void bucket_table_start_kernel(const uint32_t* __restrict__ table, uint32_t n_buckets, uint32_t stretches,
+                                          uint32_t* __restrict__ starts) {
+    const uint32_t nth = gridDim.x * blockDim.x;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t <= n_buckets; t += nth)
+        starts[t] = table[(uint64_t)t * stretches];
+}
+
+// cursor: the buckets' starts, and on return their ends; Table: the scanned
+// table of counts, which has every stretch's slots.
+template <bool Table>
 __global__ void __launch_bounds__(kBucketThreads, 1)
     bucket_scatter_kernel(const uint2* __restrict__ pairs, uint64_t n, uint64_t per, const Buckets B,
                           uint32_t* __restrict__ cursor, uint32_t* __restrict__ rec) {
@@ -163,12 +179,16 @@ __global__ void __launch_bounds__(kBucketThreads, 1)
             }
         }
     };
-    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads) s_slot[t] = 0;
-    __syncthreads();
-    each([&](uint32_t t, uint32_t) { atomicAdd(s_slot + t, 1u); });
-    __syncthreads();
-    for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads)
-        if (const uint32_t c = s_slot[t]) s_slot[t] = atomicAdd(cursor + t, c);
+    if (Table) {
+        for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads) s_slot[t] = cursor[(uint64_t)t * gridDim.x + blockIdx.x];
+    } else {
+        for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads) s_slot[t] = 0;
+        __syncthreads();
+        each([&](uint32_t t, uint32_t) { atomicAdd(s_slot + t, 1u); });
+        __syncthreads();
+        for (uint32_t t = threadIdx.x; t < B.n; t += kBucketThreads)
+            if (const uint32_t c = s_slot[t]) s_slot[t] = atomicAdd(cursor + t, c);
+    }
     __syncthreads();
     each([&](uint32_t t, uint32_t r) { rec[atomicAdd(s_slot + t, 1u)] = r; });
 }
@@ -331,20 +351,44 @@ static void converted_put(gs_ctx* ctx, gs_converted& c, bool rec) {
 
 // The two ways to fill c.d_start and c.d_rec; c.d_degree and *d_bad are zero,
 // the count pass has been launched.
-static gs_status fill_buckets(gs_ctx* ctx, const uint2* pairs, uint64_t n_pairs, const Buckets& B, uint32_t* d_bucket,
-                              const int* d_bad, gs_converted& c) {
+// The stretches of edges that a CTA counts and scatters, and whether their
+// counts are kept as a table that is scanned as a whole, so that the scatter
+// need not count again (Kronecker 22: 0.98 -> 0.81 ms; the table's scan 0.01):
+// while it is small against the edges.
+struct Stretches {
+    uint64_t per;
+    uint32_t n;
+    bool table;
+    Stretches(const gs_ctx* ctx, uint64_t n_pairs, const Buckets& B)
+        : per(std::max<uint64_t>(4 * kBucketThreads, (n_pairs + 2 * ctx->num_sms - 1) / (2 * ctx->num_sms))),
+          n((uint32_t)((n_pairs + per - 1) / per)),
+          table((uint64_t)B.n * n <= n_pairs / 16) {}
+    uint64_t counts(const Buckets& B) const { return table ? (uint64_t)B.n * n + 1 : B.n; }
+};
+
+// d_bucket: the buckets' starts, then the table or the cursors.
+static gs_status fill_buckets(gs_ctx* ctx, const uint2* pairs, uint64_t n_pairs, const Buckets& B, const Stretches& S,
+                              uint32_t* d_bucket, const int* d_bad, gs_converted& c) {
     cudaStream_t q = ctx->stream;
     uint32_t* d_cursor = d_bucket + B.n + 1;
+    uint32_t* const d_scan = S.table ? d_cursor : d_bucket;
+    const int n_scan = (int)(S.table ? S.counts(B) : B.n + 1);
     size_t scan_bytes = 0, sort_bytes = 0;
-    GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_bucket, d_bucket, B.n + 1, q));
+    GS_CHECK_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_scan, d_scan, n_scan, q));
     char* d_tmp = nullptr;
     GS_TRY(gs_pool_get(ctx, scan_bytes, (void**)&d_tmp));
-    cudaError_t e = cub::DeviceScan::ExclusiveSum(d_tmp, scan_bytes, d_bucket, d_bucket, B.n + 1, q);
+    cudaError_t e = cub::DeviceScan::ExclusiveSum(d_tmp, scan_bytes, d_scan, d_scan, n_scan, q);
     scratch_put(ctx, d_tmp, scan_bytes);
     GS_CHECK_CUDA(ctx, e);
+    if (S.table) {
+        bucket_table_start_kernel<<<64, 256, 0, q>>>(d_cursor, B.n, S.n, d_bucket);
+        GS_CHECK_CUDA(ctx, cudaGetLastError());
+        ctx->launches++;
+    } else {
+        GS_CHECK_CUDA(ctx, cudaMemcpyAsync(d_cursor, d_bucket, (size_t)B.n * 4, cudaMemcpyDeviceToDevice, q));
+    }
     GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars, d_bucket + B.n, 4, cudaMemcpyDeviceToHost, q));
     GS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 1, d_bad, sizeof(int), cudaMemcpyDeviceToHost, q));
-    GS_CHECK_CUDA(ctx, cudaMemcpyAsync(d_cursor, d_bucket, (size_t)B.n * 4, cudaMemcpyDeviceToDevice, q));
     bucket_start_kernel<<<64, 256, 0, q>>>(d_bucket, B, c.n_start - 1, c.d_start);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     GS_CHECK_CUDA(ctx, cudaStreamSynchronize(q));
@@ -356,9 +400,10 @@ static gs_status fill_buckets(gs_ctx* ctx, const uint2* pairs, uint64_t n_pairs,
     if (c.n_rec == 0) return GS_OK;
     uint32_t* d_raw = nullptr;   // the records before the sort
     GS_TRY(gs_pool_get(ctx, c.rec_bytes(), (void**)&d_raw));
-    const uint64_t per = std::max<uint64_t>(4 * kBucketThreads, (n_pairs + 2 * ctx->num_sms - 1) / (2 * ctx->num_sms));
-    bucket_scatter_kernel<<<(uint32_t)((n_pairs + per - 1) / per), kBucketThreads, (size_t)B.n * 4, q>>>(
-        pairs, n_pairs, per, B, d_cursor, d_raw);
+    if (S.table)
+        bucket_scatter_kernel<true><<<S.n, kBucketThreads, (size_t)B.n * 4, q>>>(pairs, n_pairs, S.per, B, d_cursor, d_raw);
+    else
+        bucket_scatter_kernel<false><<<S.n, kBucketThreads, (size_t)B.n * 4, q>>>(pairs, n_pairs, S.per, B, d_cursor, d_raw);
     e = cudaGetLastError();
     const int* seg = (const int*)d_bucket;   // n_rec <= 2^30
     if (e == cudaSuccess)
@@ -434,21 +479,25 @@ static gs_status convert_launch(gs_ctx* ctx, const uint32_t* d_pairs, uint64_t n
     if (p == 1 && tiles <= kMaxBuckets && n_pairs >= kBucketMinEdges && n_pairs <= (1ull << 30)) {
         while (tiles << B.bits < kEnoughBuckets && n_pairs >> (B.bits + 1) >= tiles * kBucketRecords) ++B.bits;
         B.n = (uint32_t)(tiles << B.bits);
-        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_count_kernel>(ctx->device, (int)(kMaxBuckets * 4)));
-        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_scatter_kernel>(ctx->device, (int)(kMaxBuckets * 4)));
-        const size_t bucket_bytes = ((size_t)B.n * 2 + 1) * 4;   // starts, cursors
+        const Stretches S(ctx, n_pairs, B);
+        auto* const count = S.table ? &bucket_count_kernel<true> : &bucket_count_kernel<false>;
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_count_kernel<true>>(ctx->device, (int)(kMaxBuckets * 4)));
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_count_kernel<false>>(ctx->device, (int)(kMaxBuckets * 4)));
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_scatter_kernel<true>>(ctx->device, (int)(kMaxBuckets * 4)));
+        GS_CHECK_CUDA(ctx, gs_smem_limit_once<bucket_scatter_kernel<false>>(ctx->device, (int)(kMaxBuckets * 4)));
+        const size_t bucket_bytes = ((size_t)B.n + 1 + S.counts(B)) * 4;   // starts, and the table or cursors
         uint32_t* d_bucket = nullptr;
         GS_TRY(gs_pool_get(ctx, bucket_bytes, (void**)&d_bucket));
-        cudaError_t e = cudaMemsetAsync(d_bucket, 0, ((size_t)B.n + 1) * 4, q);
+        uint32_t* const d_count = S.table ? d_bucket + B.n + 1 : d_bucket;
+        // (the table needs a zero behind it only, the counts are added to)
+        cudaError_t e = S.table ? cudaMemsetAsync(d_count + (uint64_t)B.n * S.n, 0, 4, q)
+                                : cudaMemsetAsync(d_count, 0, ((size_t)B.n + 1) * 4, q);
         if (e == cudaSuccess) {
-            const uint32_t grid = (uint32_t)std::min<uint64_t>((n_pairs + 4 * kBucketThreads - 1) / (4 * kBucketThreads),
-                                                               gs_grid_size(ctx, 1));
-            bucket_count_kernel<<<grid, kBucketThreads, (size_t)B.n * 4, q>>>(pairs, n_pairs, V, B, d_bucket, c.d_degree,
-                                                                              d_bad);
+            count<<<S.n, kBucketThreads, (size_t)B.n * 4, q>>>(pairs, n_pairs, S.per, V, B, d_count, c.d_degree, d_bad);
             ctx->launches++;
             e = cudaGetLastError();
         }
-        const gs_status st = e == cudaSuccess ? fill_buckets(ctx, pairs, n_pairs, B, d_bucket, d_bad, c)
+        const gs_status st = e == cudaSuccess ? fill_buckets(ctx, pairs, n_pairs, B, S, d_bucket, d_bad, c)
                                               : gs_cuda_fail(ctx, e, "converter");
         scratch_put(ctx, d_bucket, bucket_bytes);
         return st;

@@ -23,3 +23,9 @@ def test_convert_buckets(n, V, directed, gpu_ctx_factory, oracle_lib):
     # the converter sorts the records of a tile
     tile = np.repeat(np.arange(start.size - 1), np.diff(start).astype(np.int64))
     assert np.array_equal(grid, grid_o[np.lexsort((grid_o, tile))])
+
+
+@pytest.mark.parametrize("n, V, directed", [((1 << 24) + 5, 60_000, True), ((1 << 24) + 4099, 1 << 20, False)])
+def test_convert_scanned_counts(n, V, directed, gpu_ctx_factory, oracle_lib):
+    """Enough edges for the stretches' counts to be scanned as one table."""
+    test_convert_buckets(n, V, directed, gpu_ctx_factory, oracle_lib)

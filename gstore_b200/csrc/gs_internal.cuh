@@ -143,17 +143,21 @@ struct gs_pb_layout {
 // segments, 32 segments of one length to a slice, slices grouped into units;
 // panels are consecutive ranges of the sources in falling order of use.
 constexpr uint32_t kRlMaxPanels = 64;
+constexpr uint32_t kRlTop = 1u << 31;
 struct gs_rl_unit {              // slices [slice, slice + n_slices): `steps` x 32 16-byte groups from group off x 32 on
     uint32_t slice, n_slices, off, steps;
 };
 struct gs_rl_layout {
     uint32_t* d_ent = nullptr;       // entries, transposed by slice
-    uint32_t* d_row = nullptr;       // destination vertex of every segment (~0: none), then
+    uint32_t* d_row = nullptr;       // destination of every segment (kRlTop + i: the i-th longest row, ~0: none), then
     uint8_t* d_n4 = nullptr;         // the steps of every slice
     float* d_x = nullptr;            // x in source order, written at the start of a sweep, then
     uint32_t* d_src = nullptr;       // the vertex of every source position,
     gs_rl_unit* d_units = nullptr;   // the units,
-    unsigned int* d_tick = nullptr;  // and a unit ticket per panel and the CTAs finished
+    unsigned int* d_tick = nullptr;  // a unit ticket per panel and the CTAs finished,
+    double* d_top_sum = nullptr;     // and the sums of the n_top longest rows, zero between sweeps,
+    uint32_t* d_top = nullptr;       // and their vertices
+    uint32_t n_top = 0;
     uint32_t n_src = 0, n_panels = 0, grid = 0;
     uint32_t unit_beg[kRlMaxPanels + 1] = {};   // units of each panel
     uint32_t home_beg[kRlMaxPanels + 1] = {};   // CTAs that start on each panel

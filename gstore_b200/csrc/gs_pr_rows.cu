@@ -34,7 +34,7 @@
 //
 // Per iteration against propagation blocking (gs_pr_blocked.cu: 12.5 bytes
 // moved per entry, a shared-memory atomic per run of destinations): Kronecker
-// 20 / 24 / 26, edge factor 16: 81 / 1,045 / 5,900 us against 146 / 1,862 /
+// 20 / 24 / 26, edge factor 16: 79 / 1,027 / 5,900 us against 146 / 1,862 /
 // 8,010; the layout keeps 4.4 bytes per entry instead of 12.5.  Without hubs
 // (uniform random, 3 M vertices, 24 M entries) 153 against 100: rl_worth.
 // At Kronecker 23 the pull reads 28 % of its entries' sources through L2 and
@@ -59,6 +59,7 @@ constexpr int kRlThreads = 1024;
 constexpr uint32_t kRlWarps = kRlThreads / 32;
 constexpr uint32_t kGroups = 3 + kRlMaxPanels;   // heavy cold, light, heavy hot, then panels 1..
 constexpr uint64_t kRlPanelMin = 1ull << 19;     // entries of long rows that make a panel worth staging
+constexpr uint32_t kRlTopRows = 256;             // longest rows, whose sums are kept in 64 bits
 constexpr uint64_t kRlL2Sources = 1ull << 24;    // sources whose x (64 MB) stays in L2
 constexpr long long kWaitLimit = 1ll << 24;
 static_assert(kRlPanel % (1u << kSortSkip) == 0, "a panel boundary must survive the entry sort");
@@ -73,6 +74,8 @@ struct RlArgs {
     uint32_t n_src, n_panels;
     uint32_t unit_beg[kRlMaxPanels + 1];
     uint32_t home_beg[kRlMaxPanels + 1];
+    double* top_sum;         // [n_top]
+    uint32_t n_top;
     unsigned int* tick;      // [kRlMaxPanels] next unit of each panel, then CTAs finished; zero at launch and after it
     int* error;
 };
@@ -211,7 +214,10 @@ __global__ void __launch_bounds__(kRlThreads, 1) rl_pull_kernel(const RlArgs a) 
                     }
                     last = !__shfl_down_sync(0xFFFFFFFFu, same, 1) || lane == 31;
                 }
-                if (last && r != ~0u) atomicAdd(a.y + r, sum);
+                if (last && r != ~0u) {
+                    if (r >= kRlTop && a.n_top) atomicAdd(a.top_sum + (r - kRlTop), (double)sum);
+                    else atomicAdd(a.y + r, sum);
+                }
             }
         }
     }
@@ -219,6 +225,21 @@ __global__ void __launch_bounds__(kRlThreads, 1) rl_pull_kernel(const RlArgs a) 
     if (tid == 0 && atomicAdd(a.tick + kRlMaxPanels, 1u) == gridDim.x - 1) {
         for (int k = 0; k <= (int)kRlMaxPanels; ++k) atomicExch(a.tick + k, 0u);   // and of every CTA
     }
+}
+
+// The longest rows' sums, and zero for the next sweep.  A row of 10^5 entries
+// and more takes a hundred additions one after another, whose rounding in 32
+// bits was most of the ranks' error (2-norm against 64 bits, five iterations of
+// Kronecker 24: 1.6e-7, now 6.6e-8; 20: 7.9e-8 and 4.4e-8; propagation blocking
+// 9.8e-8 and 5.2e-8).  A launch of its own, 2-4 us: a fence and the same loop in
+// the last CTA of the sweep slowed the sweep itself (Kronecker 24: 1,024 ->
+// 1,056 us).
+__global__ void rl_top_kernel(double* __restrict__ sum, const uint32_t* __restrict__ vertex, uint32_t n,
+                              float* __restrict__ y) {
+    const uint32_t k = threadIdx.x;
+    if (k >= n) return;
+    y[vertex[k]] = (float)sum[k];
+    sum[k] = 0.0;
 }
 
 // ------------------------------------------------------------------ build --
@@ -366,12 +387,12 @@ __global__ void rl_segment_count_kernel(const uint64_t* __restrict__ keys, const
 __global__ void rl_segment_emit_kernel(const uint64_t* __restrict__ keys, const unsigned long long* __restrict__ start,
                                        uint64_t n_rows, uint64_t mask, uint32_t n_panels, uint32_t seg,
                                        const uint32_t* __restrict__ at, const uint32_t* __restrict__ vertex,
-                                       uint32_t* __restrict__ key, uint32_t* __restrict__ beg,
+                                       uint32_t n_top, uint32_t* __restrict__ key, uint32_t* __restrict__ beg,
                                        uint32_t* __restrict__ row) {
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += nth) {
         uint32_t o = at[r];
-        const uint32_t v = vertex[r];
+        const uint32_t v = r < n_top ? kRlTop + (uint32_t)r : vertex[r];
         row_segments(keys, start[r], start[r + 1], mask, n_panels, seg, [&](uint32_t g, uint64_t b, uint32_t len) {
             key[o] = g * (kRlSegMax + 1) + (kRlSegMax - len);
             beg[o] = (uint32_t)b;
@@ -617,6 +638,7 @@ gs_status build(gs_graph* g, bool* worth) {
     }));
     uint32_t n_seg = 0;
     GS_TRY(to_host(ctx, &n_seg, at + n_rows, 1));
+    const uint32_t n_top = g->N <= kRlTop ? (uint32_t)std::min<uint64_t>(n_heavy, kRlTopRows) : 0;
     uint32_t *sk0, *sk1, *si0, *si1, *sbeg, *srow;
     GS_TRY(T.get(&sk0, n_seg));
     GS_TRY(T.get(&sk1, n_seg));
@@ -625,7 +647,7 @@ gs_status build(gs_graph* g, bool* worth) {
     GS_TRY(T.get(&sbeg, n_seg));
     GS_TRY(T.get(&srow, n_seg));
     rl_segment_emit_kernel<<<grid_for(n_rows, ctx), 256, 0, ctx->stream>>>(keys, start, n_rows, mask, n_panels, seg, at,
-                                                                           row_order, sk0, sbeg, srow);
+                                                                           row_order, n_top, sk0, sbeg, srow);
     rl_iota_kernel<<<grid_for(n_seg, ctx), 256, 0, ctx->stream>>>(si0, n_seg);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     ctx->launches += 2;
@@ -717,16 +739,21 @@ gs_status build(gs_graph* g, bool* worth) {
     const uint64_t xn = (n_src + 3) & ~3ull;
     const uint64_t x_bytes = (xn * 4 + 255) & ~255ull, src_bytes = (n_src * 4 + 255) & ~255ull;
     const uint64_t unit_bytes = (units.size() * sizeof(gs_rl_unit) + 255) & ~255ull;
-    GS_TRY(gs_dev_alloc(ctx, (void**)&L.d_x, x_bytes + src_bytes + unit_bytes + (kRlMaxPanels + 1) * 4));
+    const uint64_t tick_bytes = ((kRlMaxPanels + 1) * 4 + 255) & ~255ull, top_bytes = (uint64_t)n_top * 12;
+    GS_TRY(gs_dev_alloc(ctx, (void**)&L.d_x, x_bytes + src_bytes + unit_bytes + tick_bytes + top_bytes));
     L.d_src = (uint32_t*)((char*)L.d_x + x_bytes);
     L.d_units = (gs_rl_unit*)((char*)L.d_src + src_bytes);
     L.d_tick = (unsigned int*)((char*)L.d_units + unit_bytes);
+    L.d_top_sum = (double*)((char*)L.d_tick + tick_bytes);
+    L.d_top = (uint32_t*)(L.d_top_sum + n_top);
+    L.n_top = n_top;
     if (!units.empty())
         GS_CHECK_CUDA(ctx, cudaMemcpyAsync(L.d_units, units.data(), units.size() * sizeof(gs_rl_unit),
                                            cudaMemcpyHostToDevice, ctx->stream));
     GS_CHECK_CUDA(ctx, cudaMemcpyAsync(L.d_src, src_order, n_src * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     GS_CHECK_CUDA(ctx, cudaMemsetAsync(L.d_x, 0, x_bytes, ctx->stream));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(L.d_tick, 0, (kRlMaxPanels + 1) * 4, ctx->stream));
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(L.d_tick, 0, tick_bytes + (uint64_t)n_top * 8, ctx->stream));
+    GS_CHECK_CUDA(ctx, cudaMemcpyAsync(L.d_top, row_order, (uint64_t)n_top * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     GS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     L.built = true;
     return GS_OK;
@@ -775,7 +802,7 @@ gs_status rl_launch(gs_state* s) {
     const int smem = (int)(kRlPanel + 4) * 4;
     GS_CHECK_CUDA(ctx, gs_smem_limit_once<rl_pull_kernel>(ctx->device, smem));
     RlArgs a{reinterpret_cast<const uint4*>(L.d_ent), L.d_row, L.d_n4, L.d_units, L.d_x, s->d_y, L.n_src, L.n_panels,
-             {}, {}, L.d_tick, (int*)s->d_error};
+             {}, {}, L.d_top_sum, L.n_top, L.d_tick, (int*)s->d_error};
     for (uint32_t p = 0; p <= L.n_panels; ++p) {
         a.unit_beg[p] = L.unit_beg[p];
         a.home_beg[p] = L.home_beg[p];
@@ -783,6 +810,10 @@ gs_status rl_launch(gs_state* s) {
     gs_timer_begin(ctx);
     rl_permute_kernel<<<grid_for(L.n_src, ctx), 256, 0, ctx->stream>>>(s->d_x, L.d_src, L.n_src, L.d_x);
     rl_pull_kernel<<<L.grid, kRlThreads, smem, ctx->stream>>>(a);
+    if (L.n_top) {
+        rl_top_kernel<<<1, kRlTopRows, 0, ctx->stream>>>(L.d_top_sum, L.d_top, L.n_top, s->d_y);
+        ctx->launches++;
+    }
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     ctx->launches += 2;
     // algorithmic bytes per iteration: 4E + 12V (records, x, s, inv)

@@ -335,7 +335,11 @@ struct BfsLevelOut {
 // wait instead of those, two memsets and two copies (Kronecker 16's six levels
 // 270 -> 195 us with reset and result).  A word with many new vertices gets
 // its 32 depth bytes in two 16-byte blends instead of a store per vertex (the
-// 24 M new vertices of Kronecker 26's third level: 162 -> 39 us).
+// 24 M new vertices of Kronecker 26's third level: 162 -> 39 us) -- Padded only:
+// a depth array of n_words * 32 bytes on a 16-byte boundary.  A caller's array
+// has any alignment and ends with the last vertex: new vertices alone are
+// written there, a byte each.
+template <bool Padded>
 __global__ void bfs_finalize_kernel(uint32_t* __restrict__ st, uint32_t* __restrict__ next,
                                     uint8_t* __restrict__ depth, uint64_t n_words, uint8_t next_level,
                                     unsigned long long* count, BfsLevelOut out) {
@@ -358,7 +362,7 @@ __global__ void bfs_finalize_kernel(uint32_t* __restrict__ st, uint32_t* __restr
         reinterpret_cast<uint2*>(st)[w] = make_uint2((fresh & 0xFFFFu) | (nv << 16), (nv >> 16) | (fresh & 0xFFFF0000u));
         const int n = __popc(fresh);
         local += n;
-        if (n > 4) {
+        if (Padded && n > 4) {
             uint4* d = reinterpret_cast<uint4*>(depth + w * 32);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -531,7 +535,7 @@ gs_status bfs_finalize(gs_state* s, int64_t* frontier, int* done) {
     // the level just swept, which the swap makes the next level's
     const BfsLevelOut out{(unsigned long long*)ctx->h_scalars, (const unsigned long long*)s->d_error,
                           (unsigned int*)(s->d_count + 1), s->d_act, g->nw};
-    bfs_finalize_kernel<<<blocks_for(words, ctx), 256, 0, ctx->stream>>>(
+    bfs_finalize_kernel<true><<<blocks_for(words, ctx), 256, 0, ctx->stream>>>(
         s->d_front, s->d_visited, s->d_depth, words, (uint8_t)(s->level + 1), s->d_count, out);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
@@ -575,8 +579,8 @@ gs_status bfs_level_into(gs_ctx* ctx, const gs_graph* g, uint8_t* depth, uint32_
         ctx->launches++;
     }
     const uint64_t words = g->N / 32;
-    bfs_finalize_kernel<<<blocks_for(words, ctx), 256, 0, ctx->stream>>>(st, next, depth, words, next_level, count,
-                                                                         BfsLevelOut{nullptr, nullptr, nullptr, nullptr, 0});
+    bfs_finalize_kernel<false><<<blocks_for(words, ctx), 256, 0, ctx->stream>>>(
+        st, next, depth, words, next_level, count, BfsLevelOut{nullptr, nullptr, nullptr, nullptr, 0});
     GS_CHECK_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
     return GS_OK;

@@ -451,7 +451,6 @@ __global__ void __launch_bounds__(kThreads) wk_batch_kernel(BatchArgs a) {
         for (uint64_t x = draw(); x < run_pre[n_act]; x = draw()) {
             const int ai = find_query(run_pre, n_act, x);
             const BQuery& q = a.q[act_q[ai]];
-            const gs_tile_run run = q.runs[x - run_pre[ai]];
             if (q.algo == GS_ALGO_KCORE && q.off) {
                 // the lists of the vertices removed this round, instead of every record
                 const uint64_t w0 = (x - run_pre[ai]) * kAdjWords;
@@ -493,14 +492,18 @@ __global__ void __launch_bounds__(kThreads) wk_batch_kernel(BatchArgs a) {
                 for (int k = 0; k < min(n_long, kAdjLong); ++k)
                     for (uint32_t i = long_row[k].x + threadIdx.x; i < long_row[k].y; i += kThreads)
                         atomicSub(q.deg + __ldg(q.adj + i), 1);
-            } else if (q.algo == GS_ALGO_KCORE) {
-                const KcoreOpL2 op{q.deg, q.removed, q.act + p * q.nw};
-                for (uint32_t ui = run.unit_beg + warp; ui < run.unit_end; ui += kWarps)
-                    sweep_unit(q.units[ui], q.rec, op, lane);
             } else {
-                const WccOp op{q.parent, it == 0 ? q.touched : nullptr, q.cnt + (it & 3)};
-                for (uint32_t ui = run.unit_beg + warp; ui < run.unit_end; ui += kWarps)
-                    sweep_unit(q.units[ui], q.rec, op, lane);
+                // (draws on the lists are no run numbers: a graph may have fewer runs)
+                const gs_tile_run run = q.runs[x - run_pre[ai]];
+                if (q.algo == GS_ALGO_KCORE) {
+                    const KcoreOpL2 op{q.deg, q.removed, q.act + p * q.nw};
+                    for (uint32_t ui = run.unit_beg + warp; ui < run.unit_end; ui += kWarps)
+                        sweep_unit(q.units[ui], q.rec, op, lane);
+                } else {
+                    const WccOp op{q.parent, it == 0 ? q.touched : nullptr, q.cnt + (it & 3)};
+                    for (uint32_t ui = run.unit_beg + warp; ui < run.unit_end; ui += kWarps)
+                        sweep_unit(q.units[ui], q.rec, op, lane);
+                }
             }
         }
         if (!grid_barrier(a.bar, a.err)) return;

@@ -113,10 +113,12 @@ gs_status blocked_order(gs_graph* g, uint32_t block, uint64_t* R_out, gs_tile_ru
         if (st == GS_OK) {
             block_runs_kernel<<<grid, 256, 0, q>>>(*units_out, first, run, U, *runs_out);
             e = cudaGetLastError();
-            if (e != cudaSuccess) st = gs_cuda_fail(ctx, e, "blocked order");
         }
         ctx->launches += 7;
-        // (the scratch goes back to the pool in stream order)
+        // wait: a server reads the order, and takes blocks of the pool, on streams of its own
+        const cudaError_t w = cudaStreamSynchronize(q);
+        if (e == cudaSuccess) e = w;
+        if (e != cudaSuccess && st == GS_OK) st = gs_cuda_fail(ctx, e, "blocked order");
         gs_pool_put(ctx, tmp, tmp_b);
         if (st != GS_OK) return st;
     } else {

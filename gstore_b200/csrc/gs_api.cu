@@ -26,19 +26,23 @@ gs_status gs_cuda_fail(gs_ctx* ctx, cudaError_t e, const char* what) {
 gs_status gs_dev_alloc(gs_ctx* ctx, void** ptr, size_t bytes) {
     *ptr = nullptr;
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc(ptr, bytes);
+    auto take = [&]() {
+        return ctx && bytes >= ctx->fail_least && bytes <= ctx->fail_most ? cudaErrorMemoryAllocation
+                                                                          : cudaMalloc(ptr, bytes);
+    };
+    cudaError_t e = take();
     if (e == cudaErrorMemoryAllocation && ctx && !ctx->pool_free.empty()) {
         // the pool's idle blocks hold the memory: release them, try once more
         cudaGetLastError();
         gs_pool_clear(ctx);
-        e = cudaMalloc(ptr, bytes);
+        e = take();
     }
     if (e == cudaErrorMemoryAllocation && ctx && !ctx->adj_graphs.empty()) {
         // adjacency lists only save time: drop them, try once more
         cudaGetLastError();
         gs_adj_release(ctx);
         gs_pool_clear(ctx);
-        e = cudaMalloc(ptr, bytes);
+        e = take();
     }
     if (e != cudaSuccess) {
         *ptr = nullptr;
@@ -49,6 +53,11 @@ gs_status gs_dev_alloc(gs_ctx* ctx, void** ptr, size_t bytes) {
 
 void gs_dev_free(void* ptr) {
     if (ptr) cudaFree(ptr);
+}
+
+extern "C" void gs_testing_fail_allocs(gs_ctx* ctx, uint64_t least, uint64_t most) {
+    ctx->fail_least = least;
+    ctx->fail_most = most;
 }
 
 constexpr uint64_t kPoolMaxBytes = 16ull << 30;

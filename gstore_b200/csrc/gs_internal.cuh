@@ -163,7 +163,7 @@ struct gs_rl_layout {
     uint32_t home_beg[kRlMaxPanels + 1] = {};   // CTAs that start on each panel
     uint64_t n_entries = 0;
     bool built = false;
-    bool refused = false;            // another layout sweeps this graph faster
+    bool refused = false;            // another layout sweeps this graph faster, or memory was short
 };
 
 // Adjacency lists (gs_adj.cu): the neighbours that a record leads from (in)
@@ -215,6 +215,7 @@ struct gs_ctx {
     uint64_t pool_bytes = 0;
     int adj_ctas[2] = {0, 0};        // resident CTAs per SM of the BFS and k-core launches on lists (0: not asked yet)
     std::vector<struct gs_graph*> adj_graphs;   // graphs with adjacency lists
+    uint64_t fail_least = ~0ull, fail_most = 0;   // gs_testing_fail_allocs
 };
 
 struct gs_graph {
@@ -347,6 +348,9 @@ void gs_geometry_of(uint64_t V, int directed, uint32_t* p, uint32_t* p_s, uint64
 gs_status gs_dev_alloc(gs_ctx* ctx, void** ptr, size_t bytes);
 gs_status gs_alloc_records(gs_ctx* ctx, uint32_t** ptr, uint64_t n_records);
 void gs_dev_free(void* ptr);
+// For tests of what happens when HBM is short: from now on this context's
+// device allocations of `least` to `most` bytes fail (least > most: none).
+extern "C" void gs_testing_fail_allocs(gs_ctx* ctx, uint64_t least, uint64_t most);
 // Context pool: a cached block of exactly `bytes` (rounded to 256), or a new
 // one; gs_pool_put returns it (blocks beyond kPoolMaxBytes are freed).
 gs_status gs_pool_get(gs_ctx* ctx, size_t bytes, void** out);

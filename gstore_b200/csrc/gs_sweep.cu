@@ -643,7 +643,11 @@ gs_status pr_init(gs_state* s) {
     // (rl_worth), else the propagation-blocked layout when it is worth
     // building and fits, else the row-slice layout (each built once per graph)
     if (!g->stream && g->E && !g->rl.built && !g->pb.built) {
-        if (!g->rl.refused && rl_layout_wanted(g)) GS_TRY(rl_layout_build(g));
+        if (!g->rl.refused && rl_layout_wanted(g)) {
+            const gs_status st = rl_layout_build(g);
+            if (st == GS_ERR_OOM) g->rl.refused = true;   // the others need less
+            else if (st != GS_OK) return st;
+        }
         if (!g->rl.built && !g->pr.built) {
             if (pb_layout_wanted(g)) GS_TRY(pb_layout_build(g));
             else GS_TRY(pr_layout_build(g));

@@ -1126,15 +1126,23 @@ void gs_adj_release(gs_ctx* ctx) {
     ctx->adj_graphs.clear();
 }
 
+// s->d_adj, which stays null when there is no memory for it (an allocation that
+// fails drops the lists before it gives up).
+static gs_status query_scratch(gs_state* s, size_t bytes) {
+    if (s->d_adj) return GS_OK;
+    const gs_status st = gs_state_alloc(s, &s->d_adj, bytes);
+    return st == GS_ERR_OOM ? GS_OK : st;
+}
+
 gs_status bfs_adj_run(gs_state* s, int64_t* steps) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
     const uint64_t words = g->N / 32;
     const uint32_t cap = items_cap(g);
     // both frontier queues, the long rows' chunks
-    if (!s->d_adj) GS_TRY(gs_state_alloc(s, &s->d_adj, (size_t)cap * (8 + sizeof(AdjItem))));
+    GS_TRY(query_scratch(s, (size_t)cap * (8 + sizeof(AdjItem))));
     const gs_adj& A = g->adj;
-    if (!A.built) return GS_OK;   // dropped by the allocation above
+    if (!A.built || !s->d_adj) return GS_OK;   // no room: the sweeps need none
     static_assert(sizeof(BfsCtl) <= kBfsCtlBytes, "control block");
     BfsCtl* c = (BfsCtl*)s->d_bfs_ctl;   // zero since bfs_init
     uint32_t grid = 1, block = 32;
@@ -1173,9 +1181,9 @@ gs_status kcore_adj_run(gs_state* s, int64_t* steps) {
     const uint32_t cap = (uint32_t)(n_lists(g) / kChunk + 4096);
     const size_t item_bytes = ((size_t)cap * sizeof(AdjItem) + 255) & ~(size_t)255;
     // the row chunks, the control block and the candidates
-    if (!s->d_adj) GS_TRY(gs_state_alloc(s, &s->d_adj, item_bytes + 256 + words * 4));
+    GS_TRY(query_scratch(s, item_bytes + 256 + words * 4));
     const gs_adj& A = g->adj;
-    if (!A.built) return GS_OK;   // dropped by the allocation above
+    if (!A.built || !s->d_adj) return GS_OK;   // no room: the sweeps need none
     static_assert(sizeof(KcoreCtl) <= 256, "control block");
     KcoreCtl* c = (KcoreCtl*)((char*)s->d_adj + item_bytes);
     GS_CHECK_CUDA(ctx, cudaMemsetAsync(c, 0, 256 + words * 4, ctx->stream));

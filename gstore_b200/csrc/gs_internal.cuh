@@ -489,8 +489,8 @@ constexpr size_t kBfsCtlBytes = 4352;
 bool gs_adj_ready(gs_graph* g, uint32_t sweeps);
 void gs_adj_free(gs_graph* g);
 void gs_adj_release(gs_ctx* ctx);   // drops every graph's lists (an allocation failed)
-// Whole queries from their initial state.  s->done stays false when the lists
-// were dropped meanwhile (nothing has run then).
+// Whole queries from their initial state.  s->done stays false when there was
+// no room for their scratch or the lists were dropped (nothing has run then).
 gs_status bfs_adj_run(gs_state* s, int64_t* steps);
 gs_status kcore_adj_run(gs_state* s, int64_t* steps);
 // A finished BFS: the windows that held a frontier vertex at levels 1 ..

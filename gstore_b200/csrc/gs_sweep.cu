@@ -749,8 +749,11 @@ gs_status wcc_sweep_launch(gs_state* s) {
     gs_ctx* ctx = g->ctx;
     const uint64_t bytes = 4 * g->E + 8 * g->V;
     if (s->step == 0 && g->adj.built && !g->seg.list) {
-        if (!s->d_giant) GS_TRY(gs_state_alloc(s, (void**)&s->d_giant, (g->N / 32 + 2) * 4));
-        if (g->adj.built) {   // not dropped by that allocation
+        if (!s->d_giant) {
+            const gs_status st = gs_state_alloc(s, (void**)&s->d_giant, (g->N / 32 + 2) * 4);
+            if (st != GS_OK && st != GS_ERR_OOM) return st;
+        }
+        if (g->adj.built && s->d_giant) {   // that allocation may drop the lists: then as without
             s->wcc_giant = false;
             s->wcc_touched = true;   // by its entries, every vertex of a record
             gs_timer_begin(ctx);

@@ -1137,12 +1137,15 @@ static gs_status query_scratch(gs_state* s, size_t bytes) {
 gs_status bfs_adj_run(gs_state* s, int64_t* steps) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
+    if (s->on_lists) return s->lists_status;   // failed before: a reset starts anew
     const uint64_t words = g->N / 32;
     const uint32_t cap = items_cap(g);
     // both frontier queues, the long rows' chunks
     GS_TRY(query_scratch(s, (size_t)cap * (8 + sizeof(AdjItem))));
     const gs_adj& A = g->adj;
     if (!A.built || !s->d_adj) return GS_OK;   // no room: the sweeps need none
+    s->on_lists = true;
+    s->lists_status = GS_ERR_CUDA;             // unless all goes well
     static_assert(sizeof(BfsCtl) <= kBfsCtlBytes, "control block");
     BfsCtl* c = (BfsCtl*)s->d_bfs_ctl;   // zero since bfs_init
     uint32_t grid = 1, block = 32;
@@ -1161,7 +1164,11 @@ gs_status bfs_adj_run(gs_state* s, int64_t* steps) {
     BfsCtl h;
     GS_CHECK_CUDA(ctx, cudaMemcpyAsync(&h, c, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     GS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (h.err) return gs_fail(ctx, GS_ERR_TIMEOUT, "BFS: a grid barrier wait gave up");
+    if (h.err) {
+        s->lists_status = GS_ERR_TIMEOUT;
+        return gs_fail(ctx, GS_ERR_TIMEOUT, "BFS: a grid barrier wait gave up");
+    }
+    s->lists_status = h.overflow ? GS_ERR_RANGE : GS_OK;
     s->level_counts.assign(h.total + 1, h.total + h.levels + 1);
     s->level_skip.assign(h.levels, 1);   // entries read are counted
     s->level = (uint8_t)h.levels;

@@ -476,12 +476,16 @@ gs_status bfs_init(gs_state* s) {
     s->level_skip.clear();
     s->level = 1;
     s->level_counts.clear();
+    s->on_lists = false;
+    s->lists_status = GS_OK;
     return GS_OK;
 }
 
 gs_status bfs_sweep_begin(gs_state* s) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
+    // (a query that ended well on the lists is done and is not swept again)
+    if (s->on_lists) return gs_fail(ctx, s->lists_status, "the BFS has failed: reset it first");
     GS_CHECK_CUDA(ctx, (gs_smem_limit_once<bfs_run_kernel<false, false>>(ctx->device, (int)sizeof(BfsSmem))));
     GS_CHECK_CUDA(ctx, (gs_smem_limit_once<bfs_run_kernel<true, false>>(ctx->device, (int)sizeof(BfsSmem))));
     GS_CHECK_CUDA(ctx, (gs_smem_limit_once<bfs_run_kernel<true, true>>(ctx->device, (int)sizeof(BfsSmem))));
@@ -530,6 +534,13 @@ gs_status bfs_sweep_launch(gs_state* s) {
 gs_status bfs_finalize(gs_state* s, int64_t* frontier, int* done) {
     gs_graph* g = s->g;
     gs_ctx* ctx = g->ctx;
+    if (s->on_lists) {   // one more level without a sweep finds nothing
+        if (s->lists_status != GS_OK) return gs_fail(ctx, s->lists_status, "the BFS has failed: reset it first");
+        s->level_counts.push_back(0);
+        *frontier = 0;
+        *done = 1;
+        return GS_OK;
+    }
     const uint64_t words = g->N / 32;
     // read_part_next->reset() (bfs.cpp:322-324): the kernel clears the flags of
     // the level just swept, which the swap makes the next level's

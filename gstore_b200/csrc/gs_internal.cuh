@@ -305,6 +305,8 @@ struct gs_state {
     // k-core
     int32_t* d_deg = nullptr;        // N
     uint32_t* d_kactive = nullptr;   // N/32
+    bool on_lists = false;           // BFS: gs_run took it on adjacency lists, the bitmaps are not the sweeps'
+    gs_status lists_status = GS_OK;  // and how that ended
     void* d_bfs_ctl = nullptr;       // BFS on adjacency lists: control block (kBfsCtlBytes, cleared by bfs_init)
     void* d_adj = nullptr;           // BFS, k-core on adjacency lists: queues, row chunks (k-core: control block)
     // bfs2 / traverse

@@ -529,6 +529,9 @@ extern "C" gs_status gs_convert(gs_ctx* ctx, const uint32_t* pairs, uint64_t n_p
     }
     gs_converted c;
     gs_status st = convert_launch(ctx, d_pairs, n_pairs, V, ctx->directed, c);
+    // a conversion that fails may leave kernels that read the pairs and the
+    // scratch: both are given back below (one that succeeds waits further on)
+    if (st != GS_OK) cudaStreamSynchronize(ctx->stream);
     if (d_copy) scratch_put(ctx, d_copy, n_pairs * 8);
     if (st != GS_OK) {
         converted_put(ctx, c, true);

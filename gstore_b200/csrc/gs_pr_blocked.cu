@@ -684,15 +684,22 @@ gs_status pb_pull_build(gs_graph* g, uint32_t rows, bool* fits) {
     const uint32_t many = gs_grid_size(ctx, 8);
     Temps T(ctx);
     GS_TRY(T.reserve(n_ent * 17 + n_blk * 24 + (uint64_t)R * 28 + (4ull << 20)));
-    uint32_t *count = nullptr, *most = nullptr;
-    GS_TRY(T.get(&count, g->N));
+    uint32_t* most = nullptr;
     GS_TRY(T.get(&most, 2));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(count, 0, g->N * 4, ctx->stream));
     GS_CHECK_CUDA(ctx, cudaMemsetAsync(most, 0, 8, ctx->stream));
-    pb_count_kernel<<<many, 256, 0, ctx->stream>>>(g->d_units, g->U, g->d_rec, g->directed, count);
+    const uint32_t* count = (const uint32_t*)g->d_degree;
+    if (g->directed || !g->degree_from_records) {   // else the graph has counted them
+        uint32_t* counted = nullptr;
+        GS_TRY(T.get(&counted, g->N));
+        GS_CHECK_CUDA(ctx, cudaMemsetAsync(counted, 0, g->N * 4, ctx->stream));
+        pb_count_kernel<<<many, 256, 0, ctx->stream>>>(g->d_units, g->U, g->d_rec, g->directed, counted);
+        GS_CHECK_CUDA(ctx, cudaGetLastError());
+        ctx->launches++;
+        count = counted;
+    }
     pb_bin_max_kernel<<<many, 256, 0, ctx->stream>>>(count, g->N, rows, nD, most);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
-    ctx->launches += 2;
+    ctx->launches++;
     uint32_t h_most[2];
     GS_TRY(to_host(ctx, h_most, most, 2));
     *fits = h_most[0] <= kPullRowMax && h_most[1] + 7ull * nS <= kPullVals;

@@ -243,7 +243,7 @@ __global__ void rl_top_kernel(double* __restrict__ sum, const uint32_t* __restri
 }
 
 // ------------------------------------------------------------------ build --
-// Entries per destination and per source (the half grid: the same counts).
+// Entries per destination and, with `out`, per source (the half grid: the same counts).
 __global__ void rl_count_kernel(const gs_unit* __restrict__ units, uint64_t n_units, const uint32_t* __restrict__ rec,
                                 int directed, uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
     const uint32_t lane = threadIdx.x & 31;
@@ -256,10 +256,64 @@ __global__ void rl_count_kernel(const gs_unit* __restrict__ units, uint64_t n_un
             const uint32_t r = __ldcs(rec + un.rec_beg + k);
             const uint32_t a = rb + (r & 0xFFFFu), b = cb + (r >> 16);
             atomicAdd(in + b, 1u);
-            if (directed) atomicAdd(out + a, 1u);
-            else atomicAdd(in + a, 1u);
+            if (!directed) atomicAdd(in + a, 1u);
+            else if (out) atomicAdd(out + a, 1u);
         }
     }
+}
+
+// Vertices by count: one bin per count below kSmallCounts, 64 per power of two
+// above, whose counts are added up too (no bin: zero).
+constexpr uint32_t kSmallCounts = 4096, kBigCounts = 20 * 64;
+struct RlHistogram {
+    unsigned long long big_sum[kBigCounts];
+    uint32_t small[kSmallCounts], big[kBigCounts];
+};
+
+__global__ void __launch_bounds__(1024) rl_histogram_kernel(const uint32_t* __restrict__ count, uint64_t N, RlHistogram* h) {
+    __shared__ uint32_t s[kSmallCounts];
+    for (uint32_t i = threadIdx.x; i < kSmallCounts; i += blockDim.x) s[i] = 0;
+    __syncthreads();
+    const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < N; v += nth) {
+        const uint32_t c = count[v];
+        if (c == 0) continue;
+        if (c < kSmallCounts) {
+            atomicAdd(s + c, 1u);
+        } else {
+            const uint32_t e = 31 - __clz(c), bin = (e - 12) * 64 + (c >> (e - 6) & 63);
+            atomicAdd(h->big + bin, 1u);
+            atomicAdd(h->big_sum + bin, (unsigned long long)c);
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kSmallCounts; i += blockDim.x)
+        if (s[i]) atomicAdd(h->small + i, s[i]);
+}
+
+// Entries of the k vertices of the highest counts (exact up to the part of a
+// bin above kSmallCounts that k cuts off).
+uint64_t top_entries(const RlHistogram& h, uint64_t k) {
+    uint64_t sum = 0;
+    for (uint32_t b = kBigCounts; b-- > 0 && k;) {
+        const uint64_t n = std::min<uint64_t>(k, h.big[b]);
+        if (n) sum += n == h.big[b] ? h.big_sum[b] : h.big_sum[b] / h.big[b] * n;
+        k -= n;
+    }
+    for (uint32_t c = kSmallCounts; c-- > 1 && k;) {
+        const uint64_t n = std::min<uint64_t>(k, h.small[c]);
+        sum += n * c;
+        k -= n;
+    }
+    return sum;
+}
+
+// Entries of the vertices of at least `least` < kSmallCounts.
+uint64_t long_entries(const RlHistogram& h, uint32_t least) {
+    uint64_t sum = 0;
+    for (uint32_t b = 0; b < kBigCounts; ++b) sum += h.big_sum[b];
+    for (uint32_t c = least; c < kSmallCounts; ++c) sum += (uint64_t)h.small[c] * c;
+    return sum;
 }
 
 __global__ void rl_iota_kernel(uint32_t* v, uint64_t n) {
@@ -475,8 +529,8 @@ __global__ void rl_fill_kernel(const RlGroups G, uint32_t n_slices, const uint32
 
 // Whether a pulled sweep beats what the graph would use instead, in
 // picoseconds per entry over the chip; at[0..2]: entries whose source is among
-// the first kRlPanel, all panels' and kRlL2Sources sources, at[3]: entries of
-// the long rows.  About four fifths of what the long rows have beyond panel 0
+// the first kRlPanel, all panels' and kRlL2Sources sources (panel 0, the further
+// panels of long rows, L2; the rest DRAM), at[3]: entries of the long rows.  About four fifths of what the long rows have beyond panel 0
 // falls into panels they have enough entries in.  0.9 and 5.0 fit the sweeps
 // above (Kronecker 24: 2.0 estimated, 1.8 measured; 26: 3.0 and 2.7; uniform,
 // 3 M vertices: 5.0 and 5.4); propagation blocking measured 3.5-4.9, the row
@@ -544,22 +598,53 @@ void interleave(std::vector<gs_rl_unit>& units, const RlGroups& G) {
 gs_status build(gs_graph* g, bool* worth) {
     gs_ctx* ctx = g->ctx;
     gs_rl_layout& L = g->rl;
-    Temps T(ctx);
     const uint64_t N = g->N, n_ent = g->directed ? g->E : 2 * g->E;
-    *worth = true;
     const uint32_t many = gs_grid_size(ctx, 8);
-    // two key buffers; counts, orders and ranks; cub's scratch
-    GS_TRY(T.reserve(n_ent * 16 + n_ent / 4 + N * (g->directed ? 56 : 36) + N * 12 + (8ull << 20)));
-    uint32_t *in = nullptr, *out = nullptr;
-    GS_TRY(T.get(&in, N));
-    GS_CHECK_CUDA(ctx, cudaMemsetAsync(in, 0, N * 4, ctx->stream));
-    if (g->directed) {
-        GS_TRY(T.get(&out, N));
-        GS_CHECK_CUDA(ctx, cudaMemsetAsync(out, 0, N * 4, ctx->stream));
+
+    // Entries per destination and source (what the graph counted itself is not
+    // counted again), and from their histograms whether the lists are worth
+    // building at all: nothing is reserved or sorted for a graph that another
+    // layout sweeps faster.  Making a PageRank state, uniform random graphs that
+    // end up with pulled bins, against reserving and sorting first: 24 M entries
+    // over 3 M vertices (directed) 7.1 -> 6.4 ms, 6.4 M over 400,009 5.2 -> 4.4,
+    // 64 M over 4 M 10.6 -> 8.4 (accumulated bins without an attempt: 6.7, 4.9, 10.6).
+    const bool have_out = g->degree_from_records;   // undirected: the same as in
+    const uint64_t n_counted = (g->directed ? 1 : 0) + (have_out ? 0 : 1);
+    struct Counts {
+        gs_ctx* ctx;
+        char* p = nullptr;
+        size_t bytes;
+        ~Counts() { gs_pool_put(ctx, p, bytes); }
+    } C{ctx, nullptr, 2 * sizeof(RlHistogram) + n_counted * N * 4};
+    GS_TRY(gs_pool_get(ctx, C.bytes, (void**)&C.p));
+    RlHistogram* d_hist = (RlHistogram*)C.p;
+    uint32_t* const counted = (uint32_t*)(d_hist + 2);
+    const uint32_t* const own = (const uint32_t*)g->d_degree;
+    const uint32_t* in = n_counted ? counted : own;
+    const uint32_t* out = !g->directed ? in : have_out ? own : counted + N;
+    GS_CHECK_CUDA(ctx, cudaMemsetAsync(C.p, 0, C.bytes, ctx->stream));
+    if (n_counted) {
+        rl_count_kernel<<<many, 256, 0, ctx->stream>>>(g->d_units, g->U, g->d_rec, g->directed, counted,
+                                                       have_out ? nullptr : counted + N);
+        GS_CHECK_CUDA(ctx, cudaGetLastError());
+        ctx->launches++;
     }
-    rl_count_kernel<<<many, 256, 0, ctx->stream>>>(g->d_units, g->U, g->d_rec, g->directed, in, out);
+    const uint32_t by_vertex = std::min(grid_for(N, ctx), gs_grid_size(ctx, 2));
+    rl_histogram_kernel<<<by_vertex, 1024, 0, ctx->stream>>>(in, N, d_hist);
+    if (g->directed) rl_histogram_kernel<<<by_vertex, 1024, 0, ctx->stream>>>(out, N, d_hist + 1);
     GS_CHECK_CUDA(ctx, cudaGetLastError());
-    ctx->launches++;
+    ctx->launches += g->directed ? 2 : 1;
+    std::vector<RlHistogram> hist(g->directed ? 2 : 1);
+    GS_TRY(to_host(ctx, hist.data(), d_hist, hist.size()));
+    const RlHistogram& by_use = hist.back();
+    const unsigned long long where[4] = {top_entries(by_use, kRlPanel), top_entries(by_use, (uint64_t)kRlPanel * kRlMaxPanels),
+                                         top_entries(by_use, kRlL2Sources), long_entries(hist[0], kRlHeavy)};
+    *worth = rl_worth(g, n_ent, where);
+    if (!*worth) return GS_OK;
+
+    Temps T(ctx);
+    // two key buffers; orders and ranks; cub's scratch
+    GS_TRY(T.reserve(n_ent * 16 + n_ent / 4 + N * (g->directed ? 48 : 32) + N * 12 + (8ull << 20)));
     uint32_t *row_order, *row_cnt, *row_rank, *src_order, *src_cnt, *src_rank;
     GS_TRY(sort_by_count(T, in, N, &row_order, &row_cnt, &row_rank));
     if (g->directed) {
@@ -578,19 +663,12 @@ gs_status build(gs_graph* g, bool* worth) {
     GS_TRY(to_host(ctx, h, d_res, 3));
     const uint64_t n_rows = h[0], n_src = h[1], n_heavy = h[2];
 
-    // Entries by where their source is read from: panel 0, the further panels
-    // (long rows only), L2, DRAM.
     unsigned long long* start = nullptr;
     GS_TRY(scan_counts(T, row_cnt, n_rows, n_ent, &start));
     unsigned long long* pushes = start;   // pushes by source, scanned
     if (g->directed) GS_TRY(scan_counts(T, src_cnt, n_src, n_ent, &pushes));
     GS_TRY(to_host(ctx, h, pushes + std::min<uint64_t>(kRlPanel, n_src), 1));
-    GS_TRY(to_host(ctx, h + 1, pushes + std::min<uint64_t>((uint64_t)kRlPanel * kRlMaxPanels, n_src), 1));
-    GS_TRY(to_host(ctx, h + 2, pushes + std::min<uint64_t>(kRlL2Sources, n_src), 1));
-    GS_TRY(to_host(ctx, h + 3, start + n_heavy, 1));
     const uint64_t hot = h[0];
-    *worth = rl_worth(g, n_ent, h);
-    if (!*worth) return GS_OK;
 
     // the entries, sorted by destination rank, then by source panel
     const int pos_bits = std::max(bits_for(n_src), kSortSkip);

@@ -1091,13 +1091,17 @@ void gs_adj_free(gs_graph* g) {
     A.credit = credit;
 }
 
+void gs_adj_credit(gs_graph* g, uint32_t sweeps) {
+    if (!g->adj.built && g->adj.credit < kAdjBuild) g->adj.credit += sweeps;
+}
+
 bool gs_adj_ready(gs_graph* g, uint32_t sweeps) {
     gs_adj& A = g->adj;
     if (A.built) return true;
     if (g->stream || g->E == 0 || A.refused) return false;
     gs_ctx* ctx = g->ctx;
     if (A.credit < kAdjBuild) {
-        A.credit += sweeps;
+        gs_adj_credit(g, sweeps);
         return false;
     }
     A.refused = true;   // unless all goes well

@@ -803,7 +803,7 @@ gs_status run_wk_queries(gs_batch* b, std::vector<int>& idx) {
     for (size_t s = 0; s < idx.size(); s += kMaxBatch) {
         const size_t e = std::min(idx.size(), s + kMaxBatch);
         for (size_t k = s; k < e; ++k)
-            if (b->q[idx[k]].algo == GS_ALGO_KCORE) gs_adj_ready(b->q[idx[k]].g, 4);
+            if (b->q[idx[k]].algo == GS_ALGO_KCORE) gs_adj_ready(b->q[idx[k]].g, 0);
         std::vector<BQuery> dq;
         for (size_t k = s; k < e; ++k) {
             gs_batch_query& q = b->q[idx[k]];
@@ -893,6 +893,7 @@ gs_status run_wk_queries(gs_batch* b, std::vector<int>& idx) {
             gs_batch_query& q = b->q[idx[s + k]];
             q.ran = true;
             q.sweeps = h_sweeps[k];
+            if (q.algo == GS_ALGO_KCORE) gs_adj_credit(q.g, 4);   // swept: as gs_run's
         }
     }
     return GS_OK;

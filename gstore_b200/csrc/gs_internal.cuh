@@ -489,6 +489,8 @@ bool gs_stream_read_records(const gs_graph* g, uint32_t* dst);
 constexpr uint32_t kAdjBuild = 32;
 constexpr size_t kBfsCtlBytes = 4352;
 bool gs_adj_ready(gs_graph* g, uint32_t sweeps);
+// The counting alone, for queries that have run.
+void gs_adj_credit(gs_graph* g, uint32_t sweeps);
 void gs_adj_free(gs_graph* g);
 void gs_adj_release(gs_ctx* ctx);   // drops every graph's lists (an allocation failed)
 // Whole queries from their initial state.  s->done stays false when there was

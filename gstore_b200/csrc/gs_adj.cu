@@ -1207,7 +1207,7 @@ gs_status kcore_adj_run(gs_state* s, int64_t* steps) {
     GS_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kcore_adj_kernel, dim3(grid), dim3(kThreads), args, 0,
                                                    ctx->stream));
     ctx->launches += 1;
-    gs_timer_end(ctx, GS_ALGO_KCORE, 4 * g->E + 8 * g->V);   // the records and degrees once
+    gs_timer_end(ctx, GS_ALGO_KCORE, 0);   // (the entries read depend on the rounds: no bytes claimed)
     KcoreCtl h;
     GS_CHECK_CUDA(ctx, cudaMemcpyAsync(&h, c, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     GS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -758,7 +758,7 @@ gs_status wcc_sweep_launch(gs_state* s) {
             s->wcc_touched = true;   // by its entries, every vertex of a record
             gs_timer_begin(ctx);
             GS_TRY(wcc_adj_hook(s, wcc_vote, (unsigned long long*)ctx->d_scalars));
-            gs_timer_end(ctx, GS_ALGO_WCC, bytes);
+            gs_timer_end(ctx, GS_ALGO_WCC, 0);   // (it does not read E records: no bytes claimed)
             return GS_OK;
         }
     }

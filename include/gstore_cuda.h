@@ -83,7 +83,11 @@ const char* gs_last_error(const gs_ctx* ctx);
 /* Launch all work of this context on an existing cudaStream_t (NULL = the
  * context's own stream). */
 gs_status gs_set_stream(gs_ctx* ctx, void* cuda_stream);
-/* Enable per-kernel CUDA-event timing (kind: 0 = main sweep kernel). */
+/* Enable per-kernel CUDA-event timing (kind: 0 = main sweep kernel).
+ * gs_kernel_time: what was timed since then, per algorithm.  A query on tiles
+ * adds a launch per sweep, one on adjacency lists (gs_run) a single one; bytes
+ * are the algorithmic ones of the tile sweeps (a BFS, and a query on lists, adds
+ * none: gs_bfs_records_read has a BFS's). */
 gs_status gs_profile(gs_ctx* ctx, int enable);
 gs_status gs_kernel_time(gs_ctx* ctx, int algo, uint64_t* launches, double* total_ms,
                          uint64_t* bytes);

@@ -641,7 +641,9 @@ __global__ void pb_pull_split_kernel(const uint64_t* __restrict__ keys, const ui
 
 // Gather items of the slices, whose entries start at slice_start[0 .. nS].
 // An item pays for staging its slice, so it holds 32,768 entries at least --
-// unless that leaves the CTAs less than two items each (pb_layout_build).
+// unless that leaves the CTAs less than two items each (pulled bins, uniform,
+// us per iteration: 400,009 vertices, 6.4 M entries 34.8 -> 32.8; 1,000,003 and
+// 3,000,017 vertices of 8 entries, directed, 46.2 -> 43.9 and 102.9 -> 99.5).
 std::vector<gs_pb_item1> gather_items(const gs_ctx* ctx, const std::vector<uint64_t>& slice_start) {
     const uint64_t ctas = (uint64_t)ctx->num_sms * kGatherCtas, n_pad = slice_start.back();
     const uint64_t per =
@@ -947,14 +949,14 @@ gs_status pb_layout_build(gs_graph* g) {
     // bin (pass 2), sized so that each pass has a few items per resident CTA
     // (pass 2: ~16, so that the last wave of equal items leaves few SMs idle).
     // (item boundaries stay multiples of 8 entries: every block starts on one)
-    // An item pays for staging its slice or flushing its bin, so it holds 32,768
-    // entries or 8,192 groups at least -- unless that leaves the CTAs less than
-    // two items each, where one more in every second CTA costs a third of the
-    // pass: 400,000 vertices, 6.4 M entries, no hubs: 64 -> 52 us per iteration;
-    // at 48 M and 192 M entries smaller items cost 3 and 9 %.
-    const uint64_t ctas2 = (uint64_t)ctx->num_sms * kAccCtas;
-    const uint64_t per2 = std::clamp<uint64_t>(n_groups / (ctas2 * 16),
-                                               std::clamp<uint64_t>(n_groups / (ctas2 * 2), 2048, 8192), 1ull << 19);
+    // A bin's item holds 8,192 groups at least: every further item of a bin adds
+    // its sums to y once more, in 32 bits.  2,048 groups, so that small graphs
+    // have two items per CTA, took the served ranks of Kronecker 19 from 5.5e-8
+    // to 9.4e-8 of the 64-bit ones (2-norm) and its request from 0.44 to 0.48 ms
+    // (18: 0.40 and 0.42; 17: 0.26 and 0.18); 24 M entries over 1,500,007 vertices,
+    // uniform, under a budget 106 and 119 us per iteration (400,009: 52 and 41).
+    const uint64_t per2 =
+        std::clamp<uint64_t>(n_groups / ((uint64_t)ctx->num_sms * kAccCtas * 16), 8192, 1ull << 19);
     const std::vector<gs_pb_item1> items1 = gather_items(ctx, slice_start);
     std::vector<gs_pb_item2> items2;
     for (uint32_t d = 0; d < nD; ++d) {

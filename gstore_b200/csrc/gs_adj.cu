@@ -25,8 +25,9 @@
 // graph gets them once its queries have swept it kAdjBuild times, eight BFS or
 // k-core queries or eleven WCC (gs_adj_ready: a graph that is queried only a
 // few times never pays for them, one that is queried often pays about as much
-// as it had spent by then), and only while half of the free HBM stays free.  An
-// allocation that fails drops them again (gs_adj_release).
+// as it had spent by then, in one query), and only while half of the free HBM
+// stays free.  An allocation that fails drops them for good (gs_adj_release); a
+// query that finds no room for its own scratch runs on the tiles.
 #include "gs_internal.cuh"
 #include "gs_ops.cuh"
 
@@ -809,8 +810,8 @@ __device__ __forceinline__ bool hook_l1(uint32_t* parent, uint32_t a, uint32_t b
 // The hubs hooked to their first neighbours (hubs themselves, as the lists go),
 // a neighbour a launch, each followed by pointing every hub at its root: after
 // the first round most hubs share a root and the others' hooks find it in two
-// reads.  (All four neighbours in one launch contend for the few roots left:
-// 370-405 us at Kronecker 25 instead of 245.)
+// reads.  (All links in one launch contend for the few roots left: 370-405 us at
+// Kronecker 25 instead of 245.)
 constexpr uint32_t kHubLinks = 3;
 __global__ void wcc_adj_hub_kernel(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
                                    const uint32_t* __restrict__ hubs, uint32_t n, uint32_t link, uint32_t* parent,

@@ -205,11 +205,14 @@ gs_status gs_sweep(gs_state* s, const gs_segment* segs, int n_segs);
 gs_status gs_finalize(gs_state* s, int64_t* frontier_out, int* done_out);
 /* Sweep + finalize until done, all on the device (one 8-byte read per step).
  * steps_out: number of sweeps.  Once whole queries have swept a resident graph
- * often enough (about eight BFS or k-core queries), and while HBM has room, the
- * graph also keeps its records as adjacency lists (8 bytes per record and 9
- * per vertex until gs_graph_free, dropped earlier when an allocation fails), and BFS,
- * WCC and k-core run on those: the same results and step counts, in one to
- * eight launches. */
+ * often enough (eight BFS or k-core queries, eleven WCC), and while HBM has room,
+ * the graph also keeps its records as adjacency lists (8 bytes per record and 9
+ * per vertex until gs_graph_free; dropped earlier, and not built again, when an
+ * allocation fails), and BFS, WCC and k-core run on those: the same results and
+ * step counts, in two launches for a BFS, one for a k-core and about a dozen
+ * for a WCC.  The query that finds them due builds them first, which takes
+ * about as long as seven of the queries before it (45 ms beside 6 at 2^26
+ * vertices, 16 records each). */
 gs_status gs_run(gs_state* s, int64_t* steps_out);
 
 /* Results.  BFS and BFS2: uint8 depth[V] (root 1, unreached 0, bfs.cpp:54;
@@ -248,7 +251,7 @@ gs_status gs_bfs_records_read(gs_state* s, uint64_t* read_records, int max_level
  * Runs the same sweep kernels as gs_run on a BFS state, keeps its scratch
  * state in a fixed array inside the library (about 6 MiB per GPU, for the
  * life of the process) and writes uint8 depth[V] (root 1, unreached 0) into
- * the caller's device buffer d_depth.  Limit: V <= 16777216 (else
+ * the caller's device buffer d_depth: V bytes on any boundary, no others.  Limit: V <= 16777216 (else
  * GS_ERR_RANGE).  The first call on a device looks the array up; make it
  * before any stream capture.  Calls overlapping on one GPU share the array
  * and race: issue them one after another.  d_depth is cleared and written on
